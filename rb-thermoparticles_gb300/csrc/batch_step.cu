@@ -8,6 +8,7 @@
 // count) walks the table with a grid stride, so small and large cavities share the machine without
 // per-cavity launches.
 #include "step_node.cuh"
+#include "step_node64.cuh"
 
 namespace rbtp {
 
@@ -58,9 +59,9 @@ template <int MODE, bool ODD>
 __device__ __forceinline__ void step_out(const Geo &geo, const Phys &ph, const AAOff &ao, const StepBuffers &b,
                                          int out, int ix, int iy, int iz)
 {
-    if (out == OUT_NONE) step_node<MODE, ODD, OUT_NONE, false, MODE != RBTP_STORE_F64, true>(geo, ph, b, ao, ix, iy, iz);
-    else if (out == OUT_RHO) step_node<MODE, ODD, OUT_RHO, false, MODE != RBTP_STORE_F64, true>(geo, ph, b, ao, ix, iy, iz);
-    else step_node<MODE, ODD, OUT_MACROS, false, MODE != RBTP_STORE_F64, true>(geo, ph, b, ao, ix, iy, iz);
+    if (out == OUT_NONE) step_node<MODE, ODD, OUT_NONE, false, true, true>(geo, ph, b, ao, ix, iy, iz);
+    else if (out == OUT_RHO) step_node<MODE, ODD, OUT_RHO, false, true, true>(geo, ph, b, ao, ix, iy, iz);
+    else step_node<MODE, ODD, OUT_MACROS, false, true, true>(geo, ph, b, ao, ix, iy, iz);
 }
 
 // The batched kernel carries all phase/output variants of the step body behind block-uniform
@@ -73,7 +74,8 @@ __device__ __forceinline__ void step_out(const Geo &geo, const Phys &ph, const A
 #endif
 
 template <int MODE, int TX, int TY>
-__global__ void __launch_bounds__(TX * TY, MODE == RBTP_STORE_F64 ? RBTP_STEP_MINB_F64 : RBTP_BATCH_MINB_LOW)
+__global__ void __launch_bounds__(MODE == RBTP_STORE_F64 ? 2 * TX * TY : TX * TY,
+                                  MODE == RBTP_STORE_F64 ? step64_blocks(TX * TY) : RBTP_BATCH_MINB_LOW)
     k_step_batched(const CavDesc *__restrict__ desc, const int4 *__restrict__ tiles, int ntiles)
 {
     pdl_wait();
@@ -84,12 +86,14 @@ __global__ void __launch_bounds__(TX * TY, MODE == RBTP_STORE_F64 ? RBTP_STEP_MI
     __shared__ Phys sph;
     __shared__ AAOff soff;
     constexpr int GW = sizeof(Geo) / 4, PW = sizeof(Phys) / 4, OW = sizeof(AAOff) / 4;
-    const int tid = threadIdx.y * TX + threadIdx.x;
+    constexpr bool F64 = MODE == RBTP_STORE_F64;   // two threads per node (step_node64.cuh)
+    constexpr int NT = F64 ? 2 * TX * TY : TX * TY;
+    const int tid = (threadIdx.z * TY + threadIdx.y) * TX + threadIdx.x;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int4 tl = tiles[t];
         const CavDesc &d = desc[tl.x];
         __syncthreads();   // the previous tile's readers are done
-        for (int k = tid; k < GW + PW + OW; k += TX * TY) {
+        for (int k = tid; k < GW + PW + OW; k += NT) {
             if (k < GW) reinterpret_cast<int *>(&sgeo)[k] = reinterpret_cast<const int *>(&d.geo)[k];
             else if (k < GW + PW) reinterpret_cast<int *>(&sph)[k - GW] = reinterpret_cast<const int *>(&d.ph)[k - GW];
             else reinterpret_cast<int *>(&soff)[k - GW - PW] = reinterpret_cast<const int *>(&d.aoff)[k - GW - PW];
@@ -97,7 +101,8 @@ __global__ void __launch_bounds__(TX * TY, MODE == RBTP_STORE_F64 ? RBTP_STEP_MI
         __syncthreads();
         // tile (member, x, y, z0): BATCH_TILE_Z planes from z0
         const int ix = tl.y * TX + threadIdx.x, iy = tl.z * TY + threadIdx.y, z0 = tl.w;
-        if (d.out == OUT_IDLE || ix >= sgeo.lx || iy >= sgeo.ly) continue;
+        const bool active = ix < sgeo.lx && iy < sgeo.ly;
+        if (d.out == OUT_IDLE || (!F64 && !active)) continue;
         StepBuffers b;
         b.f = d.f;
         b.g = d.g;
@@ -107,10 +112,17 @@ __global__ void __launch_bounds__(TX * TY, MODE == RBTP_STORE_F64 ? RBTP_STEP_MI
         b.fcol = nullptr; b.gcol = nullptr;
         b.status = d.status;
         const int z1 = min(z0 + BATCH_TILE_Z, sgeo.lz);
-        if (d.phase == PHASE_SWAPPED) {
-            for (int iz = z0; iz < z1; ++iz) step_out<MODE, true>(sgeo, sph, soff, b, d.out, ix, iy, iz);
-        } else {
-            for (int iz = z0; iz < z1; ++iz) step_out<MODE, false>(sgeo, sph, soff, b, d.out, ix, iy, iz);
+        const bool odd = d.phase == PHASE_SWAPPED;
+        for (int iz = z0; iz < z1; ++iz) {
+            if constexpr (F64) {
+                extern __shared__ double smem64[];
+                const int cx = min(ix, sgeo.lx - 1), cy = min(iy, sgeo.ly - 1);
+                if (odd) step_node64<TX * TY, true, false>(sgeo, sph.kd, b, d.out, cx, cy, iz, active, smem64);
+                else step_node64<TX * TY, false, false>(sgeo, sph.kd, b, d.out, cx, cy, iz, active, smem64);
+            } else {
+                if (odd) step_out<MODE, true>(sgeo, sph, soff, b, d.out, ix, iy, iz);
+                else step_out<MODE, false>(sgeo, sph, soff, b, d.out, ix, iy, iz);
+            }
         }
     }
 }
@@ -119,11 +131,25 @@ template <int MODE>
 cudaError_t launch_mode(int shape, const CavDesc *desc, const int4 *tiles, int ntiles, int grid, cudaStream_t st)
 {
     if (ntiles <= 0) return cudaSuccess;
-    if (shape == 0) return pdl_launch(k_step_batched<MODE, 32, 4>, dim3(grid), dim3(32, 4, 1), st, desc, tiles, ntiles);
-    return pdl_launch(k_step_batched<MODE, 64, 2>, dim3(grid), dim3(64, 2, 1), st, desc, tiles, ntiles);
+    constexpr bool F64 = MODE == RBTP_STORE_F64;
+    constexpr size_t smem = F64 ? step64_smem(128) : 0;
+    constexpr int TZ = F64 ? 2 : 1;
+    if (shape == 0)
+        return pdl_launch_dyn(k_step_batched<MODE, 32, 4>, dim3(grid), dim3(32, 4, TZ), smem, st, desc, tiles, ntiles);
+    return pdl_launch_dyn(k_step_batched<MODE, 64, 2>, dim3(grid), dim3(64, 2, TZ), smem, st, desc, tiles, ntiles);
 }
 
 }  // namespace
+
+cudaError_t prepare_step_batched(int mode)
+{
+    if (mode != RBTP_STORE_F64) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(k_step_batched<RBTP_STORE_F64, 32, 4>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)step64_smem(128));
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_step_batched<RBTP_STORE_F64, 64, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)step64_smem(128));
+}
 
 cudaError_t launch_batch_plan(CavDesc *desc, int n, cudaStream_t st)
 {

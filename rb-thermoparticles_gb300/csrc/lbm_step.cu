@@ -21,13 +21,14 @@
 #include <algorithm>
 
 #include "step_node.cuh"
+#include "step_node64.cuh"
 
 namespace rbtp {
 
 namespace {
 
 template <int MODE, bool ODD, int OUT>
-__global__ void __launch_bounds__(128, RBTP_STEP_MINB(MODE))
+__global__ void __launch_bounds__(128, RBTP_STEP_MINB)
     k_step(const Geo geo, const Phys ph, const StepBuffers b, const AAOff ao)
 {
     pdl_wait();
@@ -37,6 +38,21 @@ __global__ void __launch_bounds__(128, RBTP_STEP_MINB(MODE))
     const int iz = blockIdx.z;
     if (ix >= geo.lx || iy >= geo.ly) return;
     step_node<MODE, ODD, OUT>(geo, ph, b, ao, ix, iy, iz);
+}
+
+// Block (32, 1, 2): 32 nodes of a row, f and g (step_node64.cuh).
+constexpr int NODES64 = 32;
+template <bool ODD, int OUT>
+__global__ void __launch_bounds__(2 * NODES64, step64_blocks(NODES64))
+    k_step64(const Geo geo, const Phys ph, const StepBuffers b)
+{
+    extern __shared__ double smem64[];
+    pdl_wait();
+    pdl_trigger();
+    const unsigned nx = (geo.lx + NODES64 - 1) / NODES64, iy = blockIdx.x / nx;
+    const int ix = (blockIdx.x - iy * nx) * NODES64 + threadIdx.x;
+    step_node64<NODES64, ODD, OUT == OUT_MACROS_COL>(geo, ph.kd, b, OUT, min(ix, geo.lx - 1), iy, blockIdx.y,
+                                                     ix < geo.lx, smem64);
 }
 
 // Stream-only export: the post-streaming populations f(n) of the reference (its d_f / d_g after a
@@ -260,26 +276,43 @@ template <int MODE>
 cudaError_t launch_step_mode(bool odd, int out, const Geo &geo, const Phys &ph,
                              const StepBuffers &b, cudaStream_t st)
 {
-    // Warps of 32 x-nodes in one row (FP64, FP32: 16-wide blocks cost 3 % at 320x320x160, wider
-    // ones nothing).  Shifted FP16 is issue-bound: its odd steps use 16 x 2 warps, so that half as
-    // many warps hold an x-face node and take the face-tested gather and scatter (0.683 against
-    // 0.695 ms for 32-wide rows at 320x320x160); its even steps, which touch no neighbour, run
-    // best in 64-node rows (0.583 against 0.596 ms for 32-wide rows).
-    dim3 blk(32, 4, 1);
-    if (MODE == RBTP_STORE_F16S) blk = odd ? dim3(16, 8, 1) : (geo.lx % 64 == 0 ? dim3(64, 2, 1) : dim3(32, 4, 1));
-    const dim3 grd = node_grid(geo, blk);
-    const AAOff ao = make_aa_off(geo);
+    // FP64: one warp pair per block (step_node64.cuh).  FP32: warps of 32 x-nodes in one row (16-wide
+    // blocks cost 3 % at 320x320x160, wider ones nothing).  Shifted FP16 is issue-bound: its odd steps use
+    // 16 x 2 warps, so that half as many warps hold an x-face node and take the face-tested gather
+    // and scatter (0.683 against 0.695 ms for 32-wide rows at 320x320x160); its even steps, which
+    // touch no neighbour, run best in 64-node rows (0.583 against 0.596 ms for 32-wide rows).
+    if constexpr (MODE == RBTP_STORE_F64) {
+        const dim3 grd((unsigned)((geo.lx + NODES64 - 1) / NODES64) * (unsigned)geo.ly, geo.lz);
+#define RBTP_STEP_CASE(P, O)                                                                                     \
+    if (odd == P && out == O)                                                                                    \
+        return pdl_launch_dyn(k_step64<P, O>, grd, dim3(NODES64, 1, 2), step64_smem(NODES64), st, geo, ph, b);
+        RBTP_STEP_CASE(true, OUT_NONE)
+        RBTP_STEP_CASE(true, OUT_RHO)
+        RBTP_STEP_CASE(true, OUT_MACROS)
+        RBTP_STEP_CASE(true, OUT_MACROS_COL)
+        RBTP_STEP_CASE(false, OUT_NONE)
+        RBTP_STEP_CASE(false, OUT_RHO)
+        RBTP_STEP_CASE(false, OUT_MACROS)
+        RBTP_STEP_CASE(false, OUT_MACROS_COL)
+#undef RBTP_STEP_CASE
+    } else {
+        dim3 blk(32, 4, 1);
+        if (MODE == RBTP_STORE_F16S)
+            blk = odd ? dim3(16, 8, 1) : (geo.lx % 64 == 0 ? dim3(64, 2, 1) : dim3(32, 4, 1));
+        const dim3 grd = node_grid(geo, blk);
+        const AAOff ao = make_aa_off(geo);
 #define RBTP_STEP_CASE(P, O)                                                       \
     if (odd == P && out == O) return pdl_launch(k_step<MODE, P, O>, grd, blk, st, geo, ph, b, ao);
-    RBTP_STEP_CASE(true, OUT_NONE)
-    RBTP_STEP_CASE(true, OUT_RHO)
-    RBTP_STEP_CASE(true, OUT_MACROS)
-    RBTP_STEP_CASE(true, OUT_MACROS_COL)
-    RBTP_STEP_CASE(false, OUT_NONE)
-    RBTP_STEP_CASE(false, OUT_RHO)
-    RBTP_STEP_CASE(false, OUT_MACROS)
-    RBTP_STEP_CASE(false, OUT_MACROS_COL)
+        RBTP_STEP_CASE(true, OUT_NONE)
+        RBTP_STEP_CASE(true, OUT_RHO)
+        RBTP_STEP_CASE(true, OUT_MACROS)
+        RBTP_STEP_CASE(true, OUT_MACROS_COL)
+        RBTP_STEP_CASE(false, OUT_NONE)
+        RBTP_STEP_CASE(false, OUT_RHO)
+        RBTP_STEP_CASE(false, OUT_MACROS)
+        RBTP_STEP_CASE(false, OUT_MACROS_COL)
 #undef RBTP_STEP_CASE
+    }
     return cudaErrorInvalidValue;
 }
 
@@ -294,6 +327,25 @@ cudaError_t launch_step(int mode, bool odd, int out, const Geo &geo, const Phys 
     case RBTP_STORE_F16S: return launch_step_mode<RBTP_STORE_F16S>(odd, out, geo, ph, b, st);
     }
     return cudaErrorInvalidValue;
+}
+
+cudaError_t prepare_step(int mode)
+{
+    if (mode != RBTP_STORE_F64) return cudaSuccess;
+    cudaError_t e = cudaSuccess;
+    auto allow = [&](auto *kernel) {
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)step64_smem(NODES64));
+    };
+    allow(k_step64<true, OUT_NONE>);
+    allow(k_step64<true, OUT_RHO>);
+    allow(k_step64<true, OUT_MACROS>);
+    allow(k_step64<true, OUT_MACROS_COL>);
+    allow(k_step64<false, OUT_NONE>);
+    allow(k_step64<false, OUT_RHO>);
+    allow(k_step64<false, OUT_MACROS>);
+    allow(k_step64<false, OUT_MACROS_COL>);
+    return e;
 }
 
 #define RBTP_MODE_DISPATCH(mode, CALL)                                  \

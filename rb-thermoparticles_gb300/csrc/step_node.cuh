@@ -1,29 +1,21 @@
-// step_node.cuh — the per-node body of the fused stream/collide step on the in-place AA storage
-// (see lbm_step.cu for the algorithm and its reference mapping, rbtp_internal.cuh for the slots).  Included by lbm_step.cu (single cavity) and batch_step.cu
-// (many cavities over a packed tile table), which instantiate it for their launch shapes.
+// step_node.cuh — the per-node body of the fused stream/collide step of the float storage modes on
+// the in-place AA storage (see lbm_step.cu for the algorithm and its reference mapping,
+// rbtp_internal.cuh for the slots; step_node64.cuh has the FP64 step).  Included by lbm_step.cu
+// (single cavity) and batch_step.cu (many cavities over a packed tile table), which instantiate it
+// for their launch shapes.
 #pragma once
 
 #include <type_traits>
 
 #include "rbtp_internal.cuh"
 
-// Resident 128-thread blocks per SM requested from the register allocator (FP64 is bound by the
-// FP64 pipe, FP32 storage by HBM bandwidth, shifted-FP16 storage by instruction issue).  Best of
-// 4/5/6 sweeps of both step parities at 320x320x160 on GB300: 5 (<= 96 registers) for FP32 and
-// shifted FP16.  At 6 (<= 80 registers) the FP32 steps are 5 % slower and the shifted-FP16 even
-// step, spilling, takes twice as long.
-#ifndef RBTP_STEP_MINB_F64
-#define RBTP_STEP_MINB_F64 1
+// Resident 128-thread blocks per SM requested from the register allocator (FP32 storage is bound by
+// HBM bandwidth, shifted-FP16 storage by instruction issue).  Best of 4/5/6 sweeps of both step
+// parities at 320x320x160 on GB300: 5 (<= 96 registers).  At 6 (<= 80 registers) the FP32 steps are
+// 5 % slower and the shifted-FP16 even step, spilling, takes twice as long.
+#ifndef RBTP_STEP_MINB
+#define RBTP_STEP_MINB 5
 #endif
-#ifndef RBTP_STEP_MINB_F32
-#define RBTP_STEP_MINB_F32 5
-#endif
-#ifndef RBTP_STEP_MINB_F16S
-#define RBTP_STEP_MINB_F16S 5
-#endif
-#define RBTP_STEP_MINB(MODE)                                                 \
-    ((MODE) == RBTP_STORE_F64 ? RBTP_STEP_MINB_F64                           \
-                              : ((MODE) == RBTP_STORE_F32 ? RBTP_STEP_MINB_F32 : RBTP_STEP_MINB_F16S))
 
 namespace rbtp {
 
@@ -42,11 +34,8 @@ __host__ __device__ constexpr unsigned dir_mask(int axis, int sign)
 // (f_i, g_i) of one direction held as one value.  The moments and both collisions apply the same
 // operation to f and to g, pair by pair, so in the float modes the pair is a float2 and sm_100's
 // packed FP32x2 instructions (FADD2, FMUL2, FFMA2: IEEE single operations on both halves, round
-// to nearest) advance both halves in one issue slot.  FP64 keeps two scalar operations.
-template <typename R>
-struct PairOps;
-template <>
-struct PairOps<float> {
+// to nearest) advance both halves in one issue slot.
+struct PairOps {
     using T = float2;
     static __device__ __forceinline__ T mk(float a, float b) { return make_float2(a, b); }
     static __device__ __forceinline__ T add(T a, T b) { return __fadd2_rn(a, b); }
@@ -54,19 +43,6 @@ struct PairOps<float> {
     static __device__ __forceinline__ T mul(T a, T b) { return __fmul2_rn(a, b); }
     static __device__ __forceinline__ T fma(T a, T b, T c) { return __ffma2_rn(a, b, c); }
 };
-template <>
-struct PairOps<double> {
-    using T = double2;
-    static __device__ __forceinline__ T mk(double a, double b) { return make_double2(a, b); }
-    static __device__ __forceinline__ T add(T a, T b) { return make_double2(a.x + b.x, a.y + b.y); }
-    static __device__ __forceinline__ T sub(T a, T b) { return make_double2(a.x - b.x, a.y - b.y); }
-    static __device__ __forceinline__ T mul(T a, T b) { return make_double2(a.x * b.x, a.y * b.y); }
-    static __device__ __forceinline__ T fma(T a, T b, T c)
-    {
-        return make_double2(__fma_rn(a.x, b.x, c.x), __fma_rn(a.y, b.y, c.y));
-    }
-};
-
 // One node of the fused step in the in-place AA storage (StepBuffers describes the slots); shared
 // by the single-cavity kernel (lbm_step.cu) and the batched kernel (batch_step.cu).  (ix, iy, iz)
 // must lie inside the lattice.  ODD selects the odd step (gather from swapped neighbour slots,
@@ -74,7 +50,7 @@ struct PairOps<double> {
 // node's own slots only.  INTERIOR_PATH adds, for odd steps, a second copy of the gather and the
 // scatter without the box-face tests, taken by warps none of whose nodes touches a face.  It pays
 // only where the step is issue-bound (shifted-FP16 storage: odd step 0.683 against 0.84 ms without
-// it at 320x320x160); FP32 is HBM-bound (measured the same with it), FP64 FP64-pipe-bound, and
+// it at 320x320x160); FP32 is HBM-bound (measured the same with it), and
 // the batched kernel (six step variants in one kernel at 128 registers) ran 0.7 % slower with it
 // (9,010 against 9,073 MLUPS for the 256-cavity ensemble), so they leave it out.
 //
@@ -84,18 +60,17 @@ struct PairOps<double> {
 // batched kernel, whose lattice sizes are per-thread values (staged in shared memory), spills
 // 460-550 bytes per thread at 128 registers without it and none with it (+7 % ensemble
 // throughput).  The single-cavity kernel, addressing from its launch parameters, gains nothing
-// (FP32, shifted FP16) or loses half its speed (FP64), so it leaves it out.
+// and leaves it out.
 //
 // The odd-step slot offsets come from an AAOff table: the launch parameters of the single-cavity
 // kernel, a copy staged in shared memory per member in the batched kernel.
 //
 // FACE_MASK: the per-direction box-face tests read bits of two per-node masks built once from the
 // six face flags, instead of evaluating the flags' disjunction per direction.  Measured at
-// 320x320x160: FP64 odd step 13.24 against 13.41 ms, batched ensemble +0.5 % (with the staged
-// offset table); the single-cavity FP32 and shifted-FP16 odd steps run 1-2 % slower with it, so
+// 320x320x160: batched ensemble +0.5 % (with the staged offset table); the single-cavity FP32 and shifted-FP16 odd steps run 1-2 % slower with it, so
 // they keep the flag expressions.
 template <int MODE, bool ODD, int OUT, bool INTERIOR_PATH = MODE == RBTP_STORE_F16S, bool FRESH_SCATTER = false,
-          bool FACE_MASK = MODE == RBTP_STORE_F64>
+          bool FACE_MASK = false>
 __device__ __forceinline__ void step_node(const Geo &geo, const Phys &ph, const StepBuffers &b, const AAOff &ao,
                                           int ix, int iy, int iz)
 {
@@ -104,19 +79,16 @@ __device__ __forceinline__ void step_node(const Geo &geo, const Phys &ph, const 
     using R = typename ST::R;
     const long long L = geo.L;
     const long long node = (long long)iz * geo.lxy + (long long)iy * geo.lx + ix;
-    // read and written in place: no restrict (the paired float modes alias f and g)
+    // the (f, g) slots, read and written in place
     S *const fA = static_cast<S *>(b.f);
-    S *const gA = static_cast<S *>(b.g);
     // Every slot a node touches is its own slot of direction 0 plus a kernel-uniform offset: i L
     // (its own slot i), o L - off_i (odd gather), i L + off_i (odd scatter).  Addressed as one
     // per-thread base pointer plus that offset, the offset stays in the load or store instruction;
     // written as (o L + node) - off_i, each access cost two 64-bit integer additions (odd steps ran
     // 1.6-2x the even steps' instructions).
     const S *const fN = fA + node;
-    const S *const gN = gA + node;
     // the odd step's gather offset of direction I (AAOff)
     auto aa_gather = [&](auto I) -> long long { return ao.g[decltype(I)::value]; };
-    const double t0 = ph.t0;
     const bool xlo = ix == 0, xhi = ix == geo.lx - 1;
     const bool ylo = iy == 0, yhi = iy == geo.ly - 1;
     const bool zlo = iz == 0, zhi = iz == geo.lz - 1;
@@ -141,20 +113,15 @@ __device__ __forceinline__ void step_node(const Geo &geo, const Phys &ph, const 
     // its moment and collision corrections are closed-form.  The other modes work on f_i and g_i.
     constexpr bool SC = MODE == RBTP_STORE_F16S;
     const R Tc = SC ? K.tla + K.tlb * (R)ix : (R)0;   // T_c at this node
-    // (f_i, g_i) of one direction as one pair value (PairOps): a float2 in the float modes
-    using PO = PairOps<R>;
+    // (f_i, g_i) of one direction as one pair value (PairOps)
+    using PO = PairOps;
     using V = typename PO::T;
     constexpr R NZ = -(R)0;
     constexpr V NZ2 = V{NZ, NZ};
-    // both populations of a slot (one access in the paired layouts of the float modes)
-    auto ldfg = [&](const S *pf, const S *pg, double w) -> V {
-        if constexpr (SC) {
-            return __half22float2(*pf);
-        } else if constexpr (ST::PAIRED) {
-            return *pf;
-        } else {
-            return PO::mk(ST::ld_f(pf, w, t0), ST::ld_g(pg, w, t0));
-        }
+    // both populations of a slot
+    auto ldfg = [&](const S *p) -> V {
+        if constexpr (SC) return __half22float2(*p);
+        else return *p;
     };
     // F_x of the previous step, read ahead of the population gather
     using A = typename ST::A;
@@ -171,7 +138,7 @@ __device__ __forceinline__ void step_node(const Geo &geo, const Phys &ph, const 
             constexpr double w = dweight(i);
             if constexpr (!ODD || i == 0) {
                 // even step: the post-streaming f_i(x) in the natural slot (i, x)
-                fg[i] = ldfg(fN + (long long)i * L, gN + (long long)i * L, w);
+                fg[i] = ldfg(fN + (long long)i * L);
             } else {
                 // odd step: f_i(x) = f*_i(x - c_i), swapped into slot (opp(i), x - c_i); a
                 // neighbour outside the box returns f*_opp(i)(x), swapped into slot (i, x)
@@ -186,7 +153,7 @@ __device__ __forceinline__ void step_node(const Geo &geo, const Phys &ph, const 
                         src = out ? (long long)i * L : src;
                     }
                 }
-                fg[i] = ldfg(fN + src, gN + src, w);
+                fg[i] = ldfg(fN + src);
             }
         });
     };
@@ -362,7 +329,7 @@ __device__ __forceinline__ void step_node(const Geo &geo, const Phys &ph, const 
         const R wpt = w * pt;
         R gb = w * ptb - h * wpt;
         if constexpr (SC) gb += gshift;
-        if constexpr (sizeof(R) == 4 && !SC) {
+        if constexpr (!SC) {
             // Packed: S and D as (f, g) pairs.  i is the member of the pair whose first nonzero
             // component is +1 (S is even and D odd in c, so the choice is free), so the sums of
             // the (u_k, u_k) and (., v_k) pairs start without a negation and the cx terms carry
@@ -410,10 +377,8 @@ __device__ __forceinline__ void step_node(const Geo &geo, const Phys &ph, const 
                 }
             });
         } else {
-            // Scalar operations: FP64 (the pair form would spend FP64 instructions on its
-            // duplicated and zero lanes) and shifted FP16 (whose step, issue-bound at 96
-            // registers, ran 0.768 against 0.692 ms per odd step at 320x320x160 with the
-            // constant pairs)
+            // Scalar operations for shifted FP16, whose step, issue-bound at 96 registers, ran 0.768
+            // against 0.692 ms per odd step at 320x320x160 with the constant pairs
             const R ca = (R)4.5 * wk1, cb = w * k0 - h * wk1, c3 = (R)3 * wk1;
             const R ce = (R)4.5 * wG, cd = wG - h * wG, cg = (R)3 * wG;
             const R ga = (R)4.5 * wpt, gc = (R)3 * wpt;
@@ -448,18 +413,11 @@ __device__ __forceinline__ void step_node(const Geo &geo, const Phys &ph, const 
     long long snode = node;
     if constexpr (FRESH_SCATTER) asm("" : "+l"(snode));
     S *const fS = fA + snode;
-    S *const gS = gA + snode;
     // store the slot at offset rel from this node's slot of direction 0: (f, g) in the working
     // variables (shifted FP16: g relative to T_c of the slot's own node)
-    auto put = [&](long long rel, const V &v, double w) {
-        if constexpr (SC) {
-            fS[rel] = __float22half2_rn(v);
-        } else if constexpr (ST::PAIRED) {
-            fS[rel] = v;
-        } else {
-            ST::st_f(fS + rel, v.x, w, t0);
-            ST::st_g(gS + rel, v.y, w, t0);
-        }
+    auto put = [&](long long rel, const V &v) {
+        if constexpr (SC) fS[rel] = __float22half2_rn(v);
+        else fS[rel] = v;
     };
     auto scatter = [&](auto INT) {
         constexpr bool INTERIOR = decltype(INT)::value;
@@ -469,7 +427,7 @@ __device__ __forceinline__ void step_node(const Geo &geo, const Phys &ph, const 
             constexpr double w = dweight(i);
             if constexpr (!ODD || i == 0) {
                 // even step: f*_i(x) swapped into the node's own slot (opp(i), x)
-                put((long long)o * L, fg[i], w);
+                put((long long)o * L, fg[i]);
             } else {
                 // odd step: f*_i(x) streams to slot (i, x + c_i); a population leaving the box
                 // becomes the next step's f_opp(i)(x) in slot (opp(i), x): bounce-back for f, and
@@ -482,7 +440,7 @@ __device__ __forceinline__ void step_node(const Geo &geo, const Phys &ph, const 
                                        (cz == 1 && zhi) || (cz == -1 && zlo));
                 if (!out) {
                     // shifted FP16: relative to T_c(x + c_i) = T_c(x) + tlb c_ix
-                    put(aa_gather(std::integral_constant<int, o>{}), SC && cx != 0 ? PO::mk(fg[i].x, fg[i].y - K.tlb * (R)cx) : fg[i], w);
+                    put(aa_gather(std::integral_constant<int, o>{}), SC && cx != 0 ? PO::mk(fg[i].x, fg[i].y - K.tlb * (R)cx) : fg[i]);
                 } else {
                     V v = fg[i];
                     if constexpr (cx != 0) {
@@ -500,7 +458,7 @@ __device__ __forceinline__ void step_node(const Geo &geo, const Phys &ph, const 
                             }
                         }
                     }
-                    put((long long)o * L, v, w);
+                    put((long long)o * L, v);
                 }
             }
             if constexpr (OUT == OUT_MACROS_COL) {
