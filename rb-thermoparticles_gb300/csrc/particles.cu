@@ -40,14 +40,12 @@ __device__ __forceinline__ double sq3(double dx, double dy, double dz)
 // rounded double formula.
 __device__ __forceinline__ double csel(int c, double d) { return c == 0 ? 0.0 : (c > 0 ? d : -d); }
 
-__device__ __forceinline__ bool link_q(int cxi, int cyi, int czi, double x0, double y0, double z0,
-                                       double px, double py, double pz, double rsq, double &q)
+// c = |x0 - X|^2 - r^2 is the same for all directions of a node.
+__device__ __forceinline__ bool link_q(int cxi, int cyi, int czi, double dx, double dy, double dz, double c, double &q)
 {
-    const double dx = dsub(x0, px), dy = dsub(y0, py), dz = dsub(z0, pz);
     const int a = cxi * cxi + cyi * cyi + czi * czi;
     const double b = dmul(2.0, dadd(dadd(csel(cxi, dx), csel(cyi, dy)), csel(czi, dz)));
-    const double c = dsub(sq3(dx, dy, dz), rsq);
-    const double disc = dsub(dmul(b, b), dmul((double)(4 * a), c));
+    const double disc = dsub(dmul(b, b), dmul(a == 1 ? 4.0 : (a == 2 ? 8.0 : 12.0), c));
     if (disc <= 0.0) return false;
     const double num = dsub(-b, __dsqrt_rn(disc));
     q = (a == 3) ? __ddiv_rn(num, 6.0) : dmul(num, a == 1 ? 0.5 : 0.25);
@@ -80,67 +78,66 @@ __device__ __forceinline__ int ifloor(double v)
     return (int)floor(v);
 }
 
-#define PCOL(st, np, c, p) (st)[(long long)(c) * (np) + (p)]
-
-// Bounding box of links.cu:160-172: floor(p -/+ r - 0.5), clipped to the box.
-struct Box { int x0, x1, y0, y1, z0, z1; };
-
-__device__ __forceinline__ Box sphere_box(const Geo &geo, double px, double py, double pz,
-                                          double r, int pad)
+// float -> double by its bits (the conversion instruction occupies the FP64 pipe)
+__device__ __forceinline__ double widen(double v) { return v; }
+__device__ __forceinline__ double widen(float v)
 {
-    Box b;
-    b.x0 = ifloor(dsub(dsub(px, r), 0.5)) - pad;
-    b.x1 = ifloor(dsub(dadd(px, r), 0.5)) + pad;
-    b.y0 = ifloor(dsub(dsub(py, r), 0.5)) - pad;
-    b.y1 = ifloor(dsub(dadd(py, r), 0.5)) + pad;
-    b.z0 = ifloor(dsub(dsub(pz, r), 0.5)) - pad;
-    b.z1 = ifloor(dsub(dadd(pz, r), 0.5)) + pad;
-    if (b.x0 < 0) b.x0 = 0;
-    if (b.y0 < 0) b.y0 = 0;
-    if (b.z0 < 0) b.z0 = 0;
-    if (b.x1 > geo.lx - 1) b.x1 = geo.lx - 1;
-    if (b.y1 > geo.ly - 1) b.y1 = geo.ly - 1;
-    if (b.z1 > geo.lz - 1) b.z1 = geo.lz - 1;
-    return b;
+    const unsigned b = __float_as_uint(v), e = b & 0x7f800000u;
+    if (e == 0u || e == 0x7f800000u) return (double)v;   // zero, subnormal, infinite, not a number
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+}
+// Exact small integers as doubles without a conversion instruction (64 cycles of the FP64 pipe each):
+// a direction component, and the node centre ix + 1/2 (from the float of 2 ix + 1 where that is exact).
+__device__ __forceinline__ double dir_double(int c) { return __hiloint2double(c == 0 ? 0 : (c > 0 ? 0x3ff00000 : (int)0xbff00000), 0); }
+__device__ __forceinline__ double centre_double(int ix)
+{
+    if (ix >= (1 << 23)) return (double)ix + 0.5;
+    const unsigned b = __float_as_uint((float)(2 * ix + 1));
+    return __hiloint2double((int)((b >> 3) + 0x37f00000u), (int)(b << 29));
 }
 
-// Per-particle geometry (PGeo) of the current position; one thread per particle.
-__device__ __forceinline__ void pgeo_body(const Geo &geo, const Phys &ph, const PartBuffers &pb, int p)
+#define PCOL(st, np, c, p) (st)[(long long)(c) * (np) + (p)]
+
+// Bounding box of links.cu:160-172: floor(p -/+ r - 0.5), clipped to the lattice.
+struct Box { int x0, x1, y0, y1, z0, z1; };
+
+// Per-particle geometry (PGeo) of the position pos (the same in all lanes), one warp per particle: the box
+// faces, the offsets and the velocities each in a lane of their own, because a double operation
+// takes the warp 64 cycles however many lanes need it.  vel, spin: lane a < 3 holds component a.
+__device__ __forceinline__ void pgeo_warp(const Geo &geo, const Phys &ph, const PartBuffers &pb, int p,
+                                          const double (&pos)[3], double vel, double spin, double temp)
 {
-    const double *st = pb.state;
-    const double px = PCOL(st, pb.np, 0, p), py = PCOL(st, pb.np, 1, p), pz = PCOL(st, pb.np, 2, p);
-    const double r = ph.radius;
-    PGeo g;
-    const Box m = sphere_box(geo, px, py, pz, r, 0);
-    const Box l = sphere_box(geo, px, py, pz, r, 1);
-    const Box n = sphere_box(geo, px, py, pz, dadd(r, NEW_FLUID_THRESH), 1);
-    const Box *bs[3] = {&m, &l, &n};
-    int *outs[3] = {g.mbox, g.lbox, g.nbox};
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        outs[k][0] = bs[k]->x0; outs[k][1] = bs[k]->x1; outs[k][2] = bs[k]->y0;
-        outs[k][3] = bs[k]->y1; outs[k][4] = bs[k]->z0; outs[k][5] = bs[k]->z1;
+    const int lane = threadIdx.x & 31;
+    PGeo &g = pb.pgeo[p];
+    const int axis = lane < 18 ? lane % 6 / 2 : lane % 3;
+    const double x = axis == 0 ? pos[0] : (axis == 1 ? pos[1] : pos[2]);
+    if (lane < 18) {   // mbox (radius r), lbox (r, padded), nbox (r + threshold, padded): x0, x1, y0, ...
+        const double r = lane < 12 ? ph.radius : dadd(ph.radius, NEW_FLUID_THRESH);
+        const int pad = lane < 6 ? 0 : 1, n = axis == 0 ? geo.lx : (axis == 1 ? geo.ly : geo.lz);
+        const bool high = lane & 1;
+        int v = ifloor(dsub(high ? dadd(x, r) : dsub(x, r), 0.5));
+        v = high ? min(v + pad, n - 1) : max(v - pad, 0);
+        int *const box = lane < 6 ? g.mbox : (lane < 12 ? g.lbox : g.nbox);
+        box[lane % 6] = v;
+    } else if (lane < 21) {
+        const int c = ifloor(x);
+        g.ic[axis] = c;
+        g.h[axis] = 0.5f - (float)(x - (double)c);
+        g.c[axis] = (float)x;
+    } else if (lane == 21) {
+        // marking band: bounds the float error of |x - X|^2 (coordinate rounding ~6e-8 |X| per
+        // component, arithmetic rounding ~1e-7 relative)
+        const float rf2 = (float)dmul(ph.radius, ph.radius);
+        const float amax = fmaxf(fabsf((float)pos[0]), fmaxf(fabsf((float)pos[1]), fabsf((float)pos[2])));
+        g.rf2 = rf2;
+        g.band = 1.0e-3f * rf2 + 1.0e-5f * (amax + 1.0f) * ((float)ph.radius + 2.0f) + 1.0e-3f;
+        g.T = (float)temp;
+        g.momk = (float)(2.0 * ph.rho0 * 3.0);
     }
-    const double c[3] = {px, py, pz};
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        g.ic[a] = ifloor(c[a]);
-        g.h[a] = 0.5f - (float)(c[a] - (double)g.ic[a]);
-        g.c[a] = (float)c[a];
+    if (lane < 3) {
+        g.v[lane] = (float)vel;
+        g.w[lane] = (float)spin;
     }
-    // marking band: bounds the float error of |x - X|^2 (coordinate rounding ~6e-8 |X| per
-    // component, arithmetic rounding ~1e-7 relative)
-    g.rf2 = (float)dmul(r, r);
-    const float amax = fmaxf(fabsf(g.c[0]), fmaxf(fabsf(g.c[1]), fabsf(g.c[2])));
-    g.band = 1.0e-3f * g.rf2 + 1.0e-5f * (amax + 1.0f) * ((float)r + 2.0f) + 1.0e-3f;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        g.v[a] = (float)PCOL(st, pb.np, 3 + a, p);
-        g.w[a] = (float)PCOL(st, pb.np, 18 + a, p);
-    }
-    g.T = (float)PCOL(st, pb.np, 30, p);
-    g.momk = (float)(2.0 * ph.rho0 * 3.0);
-    pb.pgeo[p] = g;
 }
 
 __device__ __forceinline__ Box pgeo_box(const int (&b)[6]) { return Box{b[0], b[1], b[2], b[3], b[4], b[5]}; }
@@ -400,6 +397,11 @@ __device__ __forceinline__ void links_ibb_body(const Geo &geo, const Phys &ph, c
     const long long base = (long long)p * pb.link_cap;
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
     if constexpr (MODE == RBTP_STORE_F64) {
+        // FP64-pipe bound (64 cycles per warp instruction): the interpolations share their coefficients
+        // between f and g, factors c = -1, 0, 1 are selections, and no integer is converted (58 FP64
+        // instructions per link and a division; 382 spheres of diameter 16, 2.8 M links: 416 us, 527 us
+        // with the reference's formulas term by term)
+        const double k6 = 6.0 * ph.rho0, T2 = 2.0 * Tp;
         for (int t = chunk * IBB_THREADS + threadIdx.x; t < n; t += pb.ibb_chunks * IBB_THREADS) {
             const int x = pb.link_node[base + t];
             const int dw = pb.link_dir[base + t];
@@ -412,58 +414,57 @@ __device__ __forceinline__ void links_ibb_body(const Geo &geo, const Phys &ph, c
             const int cxi = dcx_rt(ip), cyi = dcy_rt(ip), czi = dcz_rt(ip);
             const int o = dopp_rt(ip);
             const double w = dweight_rt(ip);
-            // moving wall velocity at the intersection point (ibb.cu:33-46)
-            const double relx = ((double)ix + 0.5 + q * cxi) - px;
-            const double rely = ((double)iy + 0.5 + q * cyi) - py;
-            const double relz = ((double)iz + 0.5 + q * czi) - pz;
-            const double uwx = vx + (relz * wy - rely * wz);
-            const double uwy = vy + (relx * wz - relz * wx);
-            const double uwz = vz + (rely * wx - relx * wy);
-            const double evel = (double)cxi * uwx + (double)cyi * uwy + (double)czi * uwz;
-            const double mom = 2.0 * w * ph.rho0 * evel * 3.0;
-            const double inv_2q = (q >= 0.5) ? 0.5 / q : 0.0;
-
             // upstream node x - c_ip, in-domain fluid (flag from the link build's owner reads)
             const bool fluid1 = (dw >> LINK_UP) & 1;
             const long long x1 = (long long)x - cxi - (long long)cyi * geo.lx - (long long)czi * geo.lxy;
             const long long solid = (long long)x + cxi + (long long)cyi * geo.lx + (long long)czi * geo.lxy;
             const LinkSlots sl = link_slots(odd, L, ip, o, x, x1, solid, ix, cxi);
-
             const double f_here = fB[sl.here];
             const double g_here = gB[sl.here];
-            double fval, gval;
-            // ibb.cu:52-73 (f: q < 0.5), ibb.cu:114-128 (g: q <= 0.5)
+            // ibb.cu:52-73, 114-128: below q = 1/2 the interpolation takes the upstream population, above
+            // the opposite one (at 1/2 its coefficient is zero)
+            const bool below = q < 0.5;
+            double f_2 = 0.0, g_2 = 0.0;
             if (fluid1) {
-                if (q < 0.5) {
-                    const double f_up = fB[sl.up];
-                    fval = 2.0 * q * f_here + (1.0 - 2.0 * q) * f_up - mom;
-                } else {
-                    const double f_oc = fB[sl.opp];
-                    fval = (f_here - mom) * inv_2q + (2.0 * q - 1.0) * inv_2q * f_oc;
-                }
-            } else {
-                fval = f_here - mom;
+                f_2 = fB[below ? sl.up : sl.opp];
+                g_2 = gB[below ? sl.up : sl.opp];
             }
-            const double amp = 2.0 * w * Tp * (1.0 + rho[x]);
+            const double r = rho[x];
+            // moving wall velocity at the intersection point (ibb.cu:33-46)
+            const double relx = (centre_double(ix) + q * dir_double(cxi)) - px;
+            const double rely = (centre_double(iy) + q * dir_double(cyi)) - py;
+            const double relz = (centre_double(iz) + q * dir_double(czi)) - pz;
+            const double uwx = vx + (relz * wy - rely * wz);
+            const double uwy = vy + (relx * wz - relz * wx);
+            const double uwz = vz + (rely * wx - relx * wy);
+            const double evel = csel(cxi, uwx) + csel(cyi, uwy) + csel(czi, uwz);
+            const double mom = w * k6 * evel;
+            const double w2T = w * T2;
+            const double amp = w2T + w2T * r;
+            // f = A f_here + B f_2 - C mom, g = -(A g_here) -+ B g_2 + C amp
+            double A = 1.0, B = 0.0, Cc = 1.0;
             if (fluid1) {
-                if (q <= 0.5) {
-                    const double gu = gB[sl.up];
-                    gval = -(2.0 * q * g_here + (1.0 - 2.0 * q) * gu) + amp;
+                const double q2 = 2.0 * q;
+                if (below) {
+                    A = q2;
+                    B = 1.0 - q2;
                 } else {
-                    const double go = gB[sl.opp];
-                    gval = -g_here * inv_2q + amp * inv_2q + (2.0 * q - 1.0) * inv_2q * go;
+                    A = Cc = 0.5 / q;
+                    B = (q2 - 1.0) * A;
                 }
-            } else {
-                gval = -g_here + amp;
             }
+            const double fval = A * f_here + B * f_2 - Cc * mom;
+            const double gval = Cc * amp - A * g_here + (below ? -B : B) * g_2;
             // the population that streams into x along opp from the solid node x + c_ip: the slot
             // the next step reads as f_opp(x)
             fB[sl.out] = fval;
             gB[sl.out] = gval;
-            // ibb.cu:160-187 (force, torque about the same intersection point) and 202-204 (heat)
-            const double Fx = (cxi - uwx) * f_here - (-cxi - uwx) * fval;
-            const double Fy = (cyi - uwy) * f_here - (-cyi - uwy) * fval;
-            const double Fz = (czi - uwz) * f_here - (-czi - uwz) * fval;
+            // ibb.cu:160-187 (force c (f_here + f) - u_w (f_here - f), torque about the same
+            // intersection point) and 202-204 (heat)
+            const double fs = f_here + fval, fd = f_here - fval;
+            const double Fx = csel(cxi, fs) - uwx * fd;
+            const double Fy = csel(cyi, fs) - uwy * fd;
+            const double Fz = csel(czi, fs) - uwz * fd;
             acc[0] += Fx;
             acc[1] += Fy;
             acc[2] += Fz;
@@ -836,73 +837,66 @@ __global__ void __launch_bounds__(32 * CONTACT_WARPS) k_contact_force(const Geo 
 // ------------------------------------------------------------------------------------------------
 // History shift + Newton-Euler + temperature (pforces.cu:80-116, ibb.cu:258-262, move.cu:5-103).
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void update_body(const Phys &ph, const PartBuffers &pb, int p)
+// One warp per particle: lane a < 3 integrates axis a, lane 3 the temperature (one thread per particle
+// took 17.6 us for 1000 spheres, a chain of some 300 double operations); then the geometry cache of
+// the new position, so that the link build that follows needs no k_pgeo launch.
+constexpr int UPDATE_WARPS = 4;   // particles per 128-thread CTA
+__device__ __forceinline__ void update_warp(const Geo &geo, const Phys &ph, const PartBuffers &pb, int p)
 {
-    const int np = pb.np;
+    const int np = pb.np, lane = threadIdx.x & 31;
     double *st = pb.state;
     const double dt = 1.0;
     const double buoyancy = (1.0 - 1.0 / ph.rho_ratio) * ph.grav0;
-    // this step's hydrodynamic force, torque and heat: the link-chunk partial sums in chunk order
-    double h[7] = {0, 0, 0, 0, 0, 0, 0};
-    const double *part = pb.hpart + (long long)p * IBB_CHUNKS * 7;
-    for (int c = 0; c < pb.ibb_chunks; ++c)
-#pragma unroll
-        for (int q = 0; q < 7; ++q) h[q] += part[c * 7 + q];
-    // every column is read before any is written (the loads need not wait on the stores)
-    double col[33];
-#pragma unroll
-    for (int c = 0; c < 33; ++c) col[c] = PCOL(st, np, c, p);
-    double cf[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) cf[a] = pb.cF[a * np + p];
-    double out[33];
-#pragma unroll
-    for (int c = 0; c < 33; ++c) out[c] = col[c];
-    double vn[3], on[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
+    // this step's hydrodynamic force, torque and heat (lanes 0-6): the link-chunk partial sums in chunk order
+    double h = 0.0;
+    if (lane < 7) {
+        const double *part = pb.hpart + (long long)p * IBB_CHUNKS * 7 + lane;
+        for (int c = 0; c < pb.ibb_chunks; ++c) h += part[c * 7];
+    }
+    const double torque = __shfl_sync(0xffffffffu, h, lane < 3 ? lane + 3 : 0);
+    const double heat = __shfl_sync(0xffffffffu, h, 6);
+    double x = 0.0, vn = 0.0, on = 0.0, temp = 0.0;
+    if (lane < 3) {
         // force / torque histories: prev2 <- prev, prev <- accum, accum <- this step's sums
-        const double f_prev = col[6 + a], f_prev2 = col[9 + a];
-        const double t_prev = col[21 + a], t_prev2 = col[24 + a];
-        const double f_now = cf[a] + h[a];
-        const double t_now = h[3 + a];
-        out[12 + a] = f_prev2;
-        out[9 + a] = f_prev;
-        out[6 + a] = f_now;
-        out[27 + a] = t_prev2;
-        out[24 + a] = t_prev;
-        out[21 + a] = t_now;
+        const int a = lane;
+        const double x_old = PCOL(st, np, a, p), v_old = PCOL(st, np, 3 + a, p), f_prev = PCOL(st, np, 6 + a, p);
+        const double f_prev2 = PCOL(st, np, 9 + a, p), th_old = PCOL(st, np, 15 + a, p), o_old = PCOL(st, np, 18 + a, p);
+        const double t_prev = PCOL(st, np, 21 + a, p), t_prev2 = PCOL(st, np, 24 + a, p);
+        const double f_now = pb.cF[a * np + p] + h;
+        const double t_now = torque;
         const double combo_f = 0.5 * f_now + f_prev + 0.5 * f_prev2;
         const double combo_t = 0.5 * t_now + t_prev + 0.5 * t_prev2;
-        vn[a] = col[3 + a] + 0.5 * dt * combo_f / ph.mass;
-        if (a == 0) vn[a] += dt * buoyancy;
-        on[a] = col[18 + a] + 0.5 * dt * combo_t / ph.inertia;
+        vn = v_old + 0.5 * dt * combo_f / ph.mass;
+        if (a == 0) vn += dt * buoyancy;
+        on = o_old + 0.5 * dt * combo_t / ph.inertia;
+        x = x_old + 0.5 * dt * (vn + v_old);
+        PCOL(st, np, a, p) = x;
+        PCOL(st, np, 3 + a, p) = vn;
+        PCOL(st, np, 6 + a, p) = f_now;
+        PCOL(st, np, 9 + a, p) = f_prev;
+        PCOL(st, np, 12 + a, p) = f_prev2;
+        PCOL(st, np, 15 + a, p) = th_old + 0.5 * dt * (on + o_old);
+        PCOL(st, np, 18 + a, p) = on;
+        PCOL(st, np, 21 + a, p) = t_now;
+        PCOL(st, np, 24 + a, p) = t_prev;
+        PCOL(st, np, 27 + a, p) = t_prev2;
+    } else if (lane == 3) {
+        const double heat_prev = PCOL(st, np, 31, p);
+        temp = PCOL(st, np, 30, p) + 0.5 * dt * (heat + heat_prev) / ph.heat_cap;
+        PCOL(st, np, 30, p) = temp;
+        PCOL(st, np, 31, p) = heat;
+        PCOL(st, np, 32, p) = heat_prev;
     }
+    double pos[3];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        out[a] = col[a] + 0.5 * dt * (vn[a] + col[3 + a]);
-        out[15 + a] = col[15 + a] + 0.5 * dt * (on[a] + col[18 + a]);
-        out[3 + a] = vn[a];
-        out[18 + a] = on[a];
-    }
-    const double heat_prev = col[31];
-    const double heat = h[6];
-    out[32] = heat_prev;
-    out[31] = heat;
-    out[30] = col[30] + 0.5 * dt * (heat + heat_prev) / ph.heat_cap;
-#pragma unroll
-    for (int c = 0; c < 33; ++c) PCOL(st, np, c, p) = out[c];
+    for (int a = 0; a < 3; ++a) pos[a] = __shfl_sync(0xffffffffu, x, a);
+    pgeo_warp(geo, ph, pb, p, pos, vn, on, __shfl_sync(0xffffffffu, temp, 3));
 }
 
-// The integrator, followed by the geometry cache of the new position (same thread, same particle),
-// so the link build that follows needs no separate k_pgeo launch.
-__global__ void k_update(const Geo geo, const Phys ph, const PartBuffers pb)
+__global__ void __launch_bounds__(32 * UPDATE_WARPS) k_update(const Geo geo, const Phys ph, const PartBuffers pb)
 {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < pb.np) {
-        update_body(ph, pb, p);
-        pgeo_body(geo, ph, pb, p);
-    }
+    const int p = blockIdx.x * UPDATE_WARPS + (threadIdx.x >> 5);
+    if (p < pb.np) update_warp(geo, ph, pb, p);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -937,10 +931,13 @@ __device__ __forceinline__ void mark_body(const Geo &geo, const Phys &ph, const 
     });
 }
 
-__global__ void k_pgeo(const Geo geo, const Phys ph, const PartBuffers pb)
+__global__ void __launch_bounds__(32 * UPDATE_WARPS) k_pgeo(const Geo geo, const Phys ph, const PartBuffers pb)
 {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < pb.np) pgeo_body(geo, ph, pb, p);
+    const int p = blockIdx.x * UPDATE_WARPS + (threadIdx.x >> 5), a = min((int)(threadIdx.x & 31), 2);
+    if (p >= pb.np) return;
+    const double *st = pb.state;
+    const double pos[3] = {PCOL(st, pb.np, 0, p), PCOL(st, pb.np, 1, p), PCOL(st, pb.np, 2, p)};
+    pgeo_warp(geo, ph, pb, p, pos, PCOL(st, pb.np, 3 + a, p), PCOL(st, pb.np, 18 + a, p), PCOL(st, pb.np, 30, p));
 }
 
 template <int NT>
@@ -981,6 +978,7 @@ struct LinkShared {
     unsigned up[NT];          // directions whose neighbour is in-domain fluid (bit ip)
     int scan[NT];             // exclusive prefix of the popcounts
     int node[NT];             // lattice index of each chunk node
+    double c[NT];             // FP64: |x - X|^2 - r^2 of each chunk node with candidates
 };
 
 template <bool F32Q, int NT>
@@ -1052,6 +1050,13 @@ __device__ __forceinline__ void link_fill_body(const Geo &geo, const Phys &ph, c
                 }
             }
             my_node = (int)idx;
+            if (!F32Q && mask) {
+                const double *st = pb.state;
+                sm.c[threadIdx.x] = dsub(sq3(dsub(centre_double(ix), PCOL(st, pb.np, 0, p)),
+                                             dsub(centre_double(iy), PCOL(st, pb.np, 1, p)),
+                                             dsub(centre_double(iz), PCOL(st, pb.np, 2, p))),
+                                         dmul(ph.radius, ph.radius));
+            }
         }
         int ccount;
         const int pos = block_exclusive_scan<NT>(__popc(mask), sm.rows.wsum, ccount);
@@ -1083,9 +1088,11 @@ __device__ __forceinline__ void link_fill_body(const Geo &geo, const Phys &ph, c
                                  (float)(iy - ipy) + hy, (float)(iz - ipz) + hz, pg.rf2, q);
             if (r32 > 0) return true;
             const double *st = pb.state;
-            return link_q(dcx_rt(ip), dcy_rt(ip), dcz_rt(ip), (double)ix + 0.5, (double)iy + 0.5,
-                          (double)iz + 0.5, PCOL(st, pb.np, 0, p), PCOL(st, pb.np, 1, p),
-                          PCOL(st, pb.np, 2, p), dmul(ph.radius, ph.radius), q);
+            const double dx = dsub(centre_double(ix), PCOL(st, pb.np, 0, p));
+            const double dy = dsub(centre_double(iy), PCOL(st, pb.np, 1, p));
+            const double dz = dsub(centre_double(iz), PCOL(st, pb.np, 2, p));
+            const double c = F32Q ? dsub(sq3(dx, dy, dz), dmul(ph.radius, ph.radius)) : sm.c[lo];
+            return link_q(dcx_rt(ip), dcy_rt(ip), dcz_rt(ip), dx, dy, dz, c, q);
         };
         auto put = [&](int pos, int node, int dw, double q) {
             if (pos < pb.link_cap) {
@@ -1169,91 +1176,100 @@ __global__ void __launch_bounds__(NT) k_new_fluid(const Geo geo, const Phys ph, 
     new_fluid_body<NT>(geo, ph, pb, owner_prev, owner_cur, status, blockIdx.x, sr);
 }
 
-// Refill values (refill.cu:78-240): one warp per new-fluid node, lane ip computes population ip
-// from the post-collision populations f*_ip of previous-step fluid neighbours, as the step of the
-// given parity left them in the AA storage: after an even step in slot (opp(ip), n); after an odd
-// step in slot (ip, n + c_ip), or, where n + c_ip is outside the box, as the wall-processed
-// population in slot (opp(ip), n) (bounce-back: f*_ip itself; the Dirichlet image of g*_ip at a pure
-// x exit is inverted with the step's density at n, which the step kernel wrote to rho).
+// Refill values (refill.cu:78-240): two warps per new-fluid node, one for f and one for g; lane ip computes
+// population ip from the post-collision populations f*_ip of previous-step fluid neighbours, as the
+// step of the given parity left them in the AA storage: after an even step in slot (opp(ip), n);
+// after an odd step in slot (ip, n + c_ip), or, where n + c_ip is outside the box, as the
+// wall-processed population in slot (opp(ip), n) (bounce-back: f*_ip itself; the Dirichlet image of
+// g*_ip at a pure x exit is inverted with the step's density at n, which the step kernel wrote to
+// rho).  The kernel is a chain of loads and of FP64 additions (64 cycles each for the warp): the
+// owners of all neighbours are looked at at once, a lane each, the populations are loaded four
+// neighbours at a time, and the node macros are only formed on steps that output them.
 template <int MODE>
 __device__ __forceinline__ void refill_compute_body(const Geo &geo, const Phys &ph, const PartBuffers &pb,
                                                     const int *owner_prev, const void *f_, const void *g_,
-                                                    const double *rho, bool odd, const DevStatus *status,
-                                                    int warp0, int nwarps)
+                                                    const double *rho, bool odd, bool macros,
+                                                    const DevStatus *status, int warp0, int nwarps)
 {
     using ST = Store<MODE>;
     using S = typename ST::S;
-    const S *fB = static_cast<const S *>(f_);
-    const S *gB = static_cast<const S *>(g_);
     const int lane = threadIdx.x & 31;
     const int count = min(status->nf_count, pb.nf_cap);
     const long long L = geo.L;
     const double RT = 1.0 / 3.0;
     const double lambda0 = 1.0 - dweight(0);
-    for (int n = warp0; n < count; n += nwarps) {
+    for (int t = warp0; t < 2 * count; t += nwarps) {
+        const int n = t >> 1;
+        const bool is_g = t & 1;
+        const S *pops = static_cast<const S *>(is_g ? g_ : f_);
         const int idx = pb.nf_node[n];
         const int iz = idx / (int)geo.lxy;
         const int iy = (idx - iz * (int)geo.lxy) / geo.lx;
         const int ix = idx - iz * (int)geo.lxy - iy * geo.lx;
-        int pid = pb.nf_pid[n];
-        if (pid < 0) {
-            const int pp = owner_prev[idx];
-            if (pp >= 0) pid = pp;
+        // lane k < 27 looks at the neighbours n + c_k and n + 2 c_k of the node: bit k of near_fluid where
+        // the first was fluid, of next_fluid where the second was too
+        unsigned near_fluid, next_fluid;
+        {
+            const int k = lane < 27 ? lane : 0, c1 = dcx_rt(k), c2 = dcy_rt(k), c3 = dcz_rt(k);
+            const long long off = (long long)c3 * geo.lxy + (long long)c2 * geo.lx + c1;
+            auto fluid = [&](int m) {
+                const int x1 = ix + m * c1, y1 = iy + m * c2, z1 = iz + m * c3;
+                return k > 0 && x1 >= 0 && x1 < geo.lx && y1 >= 0 && y1 < geo.ly && z1 >= 0 && z1 < geo.lz &&
+                       owner_prev[idx + m * off] < 0;
+            };
+            const bool near = fluid(1), next = fluid(2);
+            near_fluid = __ballot_sync(0xffffffffu, near);
+            next_fluid = __ballot_sync(0xffffffffu, near && next);
         }
-        double fv = 0.0, gv = 0.0;
+        double value = 0.0;
         if (lane < 27) {
             const int ip = lane;
             const double w = dweight_rt(ip);
             const int cxp = dcx_rt(ip), cyp = dcy_rt(ip), czp = dcz_rt(ip), op = dopp_rt(ip);
-            // f*_ip and g*_ip of the previous-step fluid node n = (xn, yn, zn)
-            auto collided = [&](long long n, int xn, int yn, int zn, double &fo, double &go) {
-                if (!odd) {
-                    const long long sl = (long long)op * L + n;
-                    fo = (double)ST::ld_f(fB + sl, w, ph.t0);
-                    go = (double)ST::ld_g(gB + sl, w, gshift(ph, xn));
-                    return;
-                }
-                const int xd = xn + cxp, yd = yn + cyp, zd = zn + czp;
-                if (xd >= 0 && xd < geo.lx && yd >= 0 && yd < geo.ly && zd >= 0 && zd < geo.lz) {
-                    const long long sl = (long long)ip * L + (long long)zd * geo.lxy + (long long)yd * geo.lx + xd;
-                    fo = (double)ST::ld_f(fB + sl, w, ph.t0);
-                    go = (double)ST::ld_g(gB + sl, w, gshift(ph, xd));
-                    return;
-                }
-                const long long sl = (long long)op * L + n;
-                fo = (double)ST::ld_f(fB + sl, w, ph.t0);
-                go = (double)ST::ld_g(gB + sl, w, gshift(ph, xn));
-                const bool ox = xd < 0 || xd >= geo.lx, oyz = yd < 0 || yd >= geo.ly || zd < 0 || zd >= geo.lz;
-                if (ox && !oyz) go = wall_image(go, w, xd < 0 ? ph.thot : ph.tcold, rho[n]);
+            auto load = [&](long long slot, int xs) {
+                return widen(is_g ? ST::ld_g(pops + slot, w, gshift(ph, xs)) : ST::ld_f(pops + slot, w, ph.t0));
             };
-            double tf = 0.0, tg = 0.0;
-            int sc = 0;
-            for (int ip2 = 1; ip2 < 27; ++ip2) {
-                const int cx2 = dcx_rt(ip2), cy2 = dcy_rt(ip2), cz2 = dcz_rt(ip2);
-                const int x1 = ix + cx2, y1 = iy + cy2, z1 = iz + cz2;
-                if (x1 < 0 || x1 >= geo.lx || y1 < 0 || y1 >= geo.ly || z1 < 0 || z1 >= geo.lz) continue;
-                const long long i1 = (long long)z1 * geo.lxy + (long long)y1 * geo.lx + x1;
-                if (owner_prev[i1] >= 0) continue;
-                const int x2 = ix + 2 * cx2, y2 = iy + 2 * cy2, z2 = iz + 2 * cz2;
-                const bool in2 = x2 >= 0 && x2 < geo.lx && y2 >= 0 && y2 < geo.ly && z2 >= 0 && z2 < geo.lz;
-                double f1, g1;
-                collided(i1, x1, y1, z1, f1, g1);
-                if (in2) {
-                    const long long i2 = (long long)z2 * geo.lxy + (long long)y2 * geo.lx + x2;
-                    if (owner_prev[i2] < 0) {
-                        double f2, g2;
-                        collided(i2, x2, y2, z2, f2, g2);
-                        tf += 2.0 * f1 - f2;
-                        tg += 2.0 * g1 - g2;
-                        ++sc;
-                        continue;
-                    }
+            // f*_ip or g*_ip of the previous-step fluid node n = (xn, yn, zn)
+            auto collided = [&](long long n, int xn, int yn, int zn) -> double {
+                if (!odd) return load((long long)op * L + n, xn);
+                const int xd = xn + cxp, yd = yn + cyp, zd = zn + czp;
+                if (xd >= 0 && xd < geo.lx && yd >= 0 && yd < geo.ly && zd >= 0 && zd < geo.lz)
+                    return load((long long)ip * L + (long long)zd * geo.lxy + (long long)yd * geo.lx + xd, xd);
+                double v = load((long long)op * L + n, xn);
+                const bool ox = xd < 0 || xd >= geo.lx, oyz = yd < 0 || yd >= geo.ly || zd < 0 || zd >= geo.lz;
+                if (is_g && ox && !oyz) v = wall_image(v, w, xd < 0 ? ph.thot : ph.tcold, rho[n]);
+                return v;
+            };
+            const int sc = __popc(near_fluid);
+            for (unsigned m = near_fluid; m;) {   // ascending neighbours
+                double v1[4], v2[4];
+                unsigned mm = m;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (!mm) break;
+                    const int ip2 = __ffs((int)mm) - 1;
+                    mm &= mm - 1;
+                    const int cx2 = dcx_rt(ip2), cy2 = dcy_rt(ip2), cz2 = dcz_rt(ip2);
+                    const long long off = (long long)cz2 * geo.lxy + (long long)cy2 * geo.lx + cx2;
+                    v1[k] = collided(idx + off, ix + cx2, iy + cy2, iz + cz2);
+                    if (next_fluid >> ip2 & 1u)
+                        v2[k] = collided(idx + 2 * off, ix + 2 * cx2, iy + 2 * cy2, iz + 2 * cz2);
                 }
-                tf += f1;
-                tg += g1;
-                ++sc;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (!m) break;
+                    const int ip2 = __ffs((int)m) - 1;
+                    m &= m - 1;
+                    if (next_fluid >> ip2 & 1u) value += 2.0 * v1[k] - v2[k];
+                    else value += v1[k];
+                }
             }
             if (sc == 0) {
+                int pid = pb.nf_pid[n];
+                if (pid < 0) {
+                    const int pp = owner_prev[idx];
+                    if (pp >= 0) pid = pp;
+                }
                 double px = 0, py = 0, pz = 0, vx = 0, vy = 0, vz = 0, wx = 0, wy = 0, wz = 0;
                 double tT = ph.t0;
                 const double *st = pb.state;
@@ -1274,49 +1290,39 @@ __device__ __forceinline__ void refill_compute_body(const Geo &geo, const Phys &
                 // refill.cu:196-201: eu is c.u without the 1/RT factor
                 const double eu = dcx_rt(ip) * u + dcy_rt(ip) * v + dcz_rt(ip) * ww;
                 const double uv = (u * u + v * v + ww * ww) / RT;
-                tf = w * (r + eu + 0.5 * (eu * eu - uv));
-                tg = w * tT * (1.0 + eu + 0.5 * (eu * eu - uv));
-                if (ip == 0) tg -= lambda0 * tT * r;
-                else tg += w * tT * r;
-                sc = 1;
+                if (!is_g) {
+                    value = w * (r + eu + 0.5 * (eu * eu - uv));
+                } else {
+                    value = w * tT * (1.0 + eu + 0.5 * (eu * eu - uv));
+                    if (ip == 0) value -= lambda0 * tT * r;
+                    else value += w * tT * r;
+                }
             }
-            const double inv = 1.0 / (double)sc;
-            fv = tf * inv;
-            gv = tg * inv;
-            pb.nf_val[(long long)n * 54 + ip] = fv;
-            pb.nf_val[(long long)n * 54 + 27 + ip] = gv;
+            const double inv = 1.0 / (double)max(sc, 1);
+            value *= inv;
+            pb.nf_val[(long long)n * 54 + (is_g ? 27 : 0) + ip] = value;
         }
-        // node macros in population order (refill.cu:226-239), lane 0
-        double rho_loc = 0, mx = 0, my = 0, mz = 0, phi_loc = 0;
+        if (!macros) continue;
+        // node macros in population order (refill.cu:226-239): lane 0 sums rho or phi, lanes 1-3 the momentum
+        double sum = 0.0;
         for (int ip = 0; ip < 27; ++ip) {
-            const double a = __shfl_sync(0xffffffffu, fv, ip);
-            const double c = __shfl_sync(0xffffffffu, gv, ip);
-            rho_loc += a;
-            mx += dcx_rt(ip) * a;
-            my += dcy_rt(ip) * a;
-            mz += dcz_rt(ip) * a;
-            phi_loc += c;
+            const double a = __shfl_sync(0xffffffffu, value, ip);
+            const int k = lane == 1 ? dcx_rt(ip) : (lane == 2 ? dcy_rt(ip) : (lane == 3 ? dcz_rt(ip) : 1));
+            if (k) sum += k > 0 ? a : -a;
         }
-        if (lane == 0) {
-            double *m = pb.nf_mac + (long long)n * 5;
-            m[0] = rho_loc;
-            if (rho_loc > 1e-12) {
-                const double inv_rho = 1.0 / rho_loc;
-                m[1] = mx * inv_rho; m[2] = my * inv_rho; m[3] = mz * inv_rho;
-            } else {
-                m[1] = 0.0; m[2] = 0.0; m[3] = 0.0;
-            }
-            m[4] = phi_loc;
-        }
+        const double rho_loc = __shfl_sync(0xffffffffu, sum, 0);
+        double *const m = pb.nf_mac + (long long)n * 5;
+        if (lane == 0) m[is_g ? 4 : 0] = sum;
+        else if (!is_g && lane < 4) m[lane] = rho_loc > 1e-12 ? sum * (1.0 / rho_loc) : 0.0;
     }
 }
 
 template <int MODE>
 __global__ void k_refill_compute(const Geo geo, const Phys ph, const PartBuffers pb,
                                  const int *owner_prev, const void *f_, const void *g_, const double *rho,
-                                 bool odd, const DevStatus *status)
+                                 bool odd, bool macros, const DevStatus *status)
 {
-    refill_compute_body<MODE>(geo, ph, pb, owner_prev, f_, g_, rho, odd, status,
+    refill_compute_body<MODE>(geo, ph, pb, owner_prev, f_, g_, rho, odd, macros, status,
                               (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5);
 }
 
@@ -1432,7 +1438,7 @@ cudaError_t launch_contacts(const Geo &geo, const Phys &ph, const PartBuffers &p
 cudaError_t launch_update(const Geo &geo, const Phys &ph, const PartBuffers &pb, cudaStream_t st)
 {
     if (pb.np <= 0) return cudaSuccess;
-    k_update<<<(pb.np + 127) / 128, 128, 0, st>>>(geo, ph, pb);
+    k_update<<<(pb.np + UPDATE_WARPS - 1) / UPDATE_WARPS, 32 * UPDATE_WARPS, 0, st>>>(geo, ph, pb);
     return cudaGetLastError();
 }
 
@@ -1442,7 +1448,7 @@ cudaError_t launch_mark(const Geo &geo, const Phys &ph, const PartBuffers &pb, i
     cudaError_t e = cudaMemsetAsync(owner_out, 0xFF, sizeof(int) * (size_t)geo.L, st);
     if (e) return e;
     if (pb.np <= 0) return cudaSuccess;
-    if (pgeo) k_pgeo<<<(pb.np + 127) / 128, 128, 0, st>>>(geo, ph, pb);
+    if (pgeo) k_pgeo<<<(pb.np + UPDATE_WARPS - 1) / UPDATE_WARPS, 32 * UPDATE_WARPS, 0, st>>>(geo, ph, pb);
     if (pb.np < PARTICLES_WIDE) k_mark<LINK_WIDE><<<pb.np, LINK_WIDE, 0, st>>>(geo, ph, pb, owner_out);
     else k_mark<LINK_NARROW><<<pb.np, LINK_NARROW, 0, st>>>(geo, ph, pb, owner_out);
     return cudaGetLastError();
@@ -1476,7 +1482,7 @@ cudaError_t launch_refill(int mode, const Geo &geo, const Phys &ph, const PartBu
         k_new_fluid<LINK_WIDE><<<pb.np, LINK_WIDE, 0, st>>>(geo, ph, pb, owner_prev, owner_cur, status);
     else
         k_new_fluid<LINK_NARROW><<<pb.np, LINK_NARROW, 0, st>>>(geo, ph, pb, owner_prev, owner_cur, status);
-    RBTP_MODE_DISPATCH(mode, (k_refill_compute<M><<<152, 256, 0, st>>>(geo, ph, pb, owner_prev, f, g, rho, odd, status)));
+    RBTP_MODE_DISPATCH(mode, (k_refill_compute<M><<<152, 256, 0, st>>>(geo, ph, pb, owner_prev, f, g, rho, odd, macros, status)));
     RBTP_MODE_DISPATCH(mode, (k_refill_scatter<M><<<152, 256, 0, st>>>(geo, ph, pb, f, g, faux, rho_wall, macros, rho, ux, uy, uz, phi, status, odd)));
     return cudaGetLastError();
 }
@@ -1565,17 +1571,16 @@ __global__ void __launch_bounds__(32 * CONTACT_WARPS) k_contact_force_b(const Ca
     contact_force_body(d.geo, d.ph, d.pb, d.status, mp.y, cand[w], ncand[w]);
 }
 
-__global__ void k_update_b(const CavDesc *desc, const int2 *pmap, int total)
+__global__ void __launch_bounds__(32 * UPDATE_WARPS) k_update_b(const CavDesc *desc, const int2 *pmap, int total)
 {
     pdl_wait();
     pdl_trigger();
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    const int g = blockIdx.x * UPDATE_WARPS + (threadIdx.x >> 5);
     if (g >= total) return;
     const int2 mp = pmap[g];
     const CavDesc &d = desc[mp.x];
     if (d.out == OUT_IDLE) return;
-    update_body(d.ph, d.pb, mp.y);
-    pgeo_body(d.geo, d.ph, d.pb, mp.y);   // geometry cache of the new position
+    update_warp(d.geo, d.ph, d.pb, mp.y);
 }
 
 __global__ void k_owner_fill_b(const CavDesc *desc, const int *pmem)
@@ -1637,7 +1642,7 @@ __global__ void k_refill_compute_b(const CavDesc *desc, const int *pmem)
     const CavDesc &d = desc[pmem[blockIdx.y]];
     if (d.out == OUT_IDLE) return;
     refill_compute_body<MODE>(d.geo, d.ph, d.pb, d.owner[d.ocur], d.f, d.g, d.rho, d.phase == PHASE_SWAPPED,
-                              d.status, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+                              d.out == OUT_MACROS, d.status, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
                               (gridDim.x * blockDim.x) >> 5);
 }
 
@@ -1677,7 +1682,7 @@ cudaError_t particles_batched_mode(const CavDesc *desc, const int2 *pmap, int to
     if ((e = cudaEventRecord(ev_join, side)) != cudaSuccess) return e;
     RBTP_PDL(k_links_ibb_b<MODE>, dim3(ncmap), dim3(IBB_THREADS), st, desc, pmap, cmap);
     if ((e = cudaStreamWaitEvent(st, ev_join, 0)) != cudaSuccess) return e;
-    RBTP_PDL(k_update_b, dim3(bl), dim3(t), st, desc, pmap, total);
+    RBTP_PDL(k_update_b, dim3((total + UPDATE_WARPS - 1) / UPDATE_WARPS), dim3(32 * UPDATE_WARPS), st, desc, pmap, total);
     RBTP_PDL(k_owner_fill_b, dim3(64, npmem), dim3(256), st, desc, pmem);
     if (total < PARTICLES_WIDE) {
         RBTP_PDL(k_mark_b<LINK_WIDE>, dim3(total), dim3(LINK_WIDE), st, desc, pmap);
@@ -1688,7 +1693,7 @@ cudaError_t particles_batched_mode(const CavDesc *desc, const int2 *pmap, int to
         RBTP_PDL(k_link_fill_b<MODE != RBTP_STORE_F64, LINK_NARROW>, dim3(total), dim3(LINK_NARROW), st, desc, pmap);
         RBTP_PDL(k_new_fluid_b<LINK_NARROW>, dim3(total), dim3(LINK_NARROW), st, desc, pmap);
     }
-    RBTP_PDL(k_refill_compute_b<MODE>, dim3(8, npmem), dim3(256), st, desc, pmem);
+    RBTP_PDL(k_refill_compute_b<MODE>, dim3(16, npmem), dim3(256), st, desc, pmem);
     RBTP_PDL(k_refill_scatter_b<MODE>, dim3(8, npmem), dim3(256), st, desc, pmem);
 #undef RBTP_PDL
     return cudaGetLastError();

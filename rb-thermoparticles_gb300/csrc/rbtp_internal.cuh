@@ -372,7 +372,7 @@ constexpr int ibb_chunks_for(long long link_cap)
     return link_cap <= 2048 ? 1 : (link_cap >= 2048LL * IBB_CHUNKS ? IBB_CHUNKS : (int)((link_cap + 2047) / 2048));
 }
 
-// Per-particle geometry derived once per link build from the FP64 position (one thread per
+// Per-particle geometry derived once per link build from the FP64 position (one warp per
 // particle), so that the per-particle CTAs spend no FP64 work on their setup: the integer boxes of
 // marking (radius r), link fill (r, padded by 1) and new-fluid detection (r + 1.76..., padded by 1),
 // the integer part of the centre and 1/2 minus its fraction (exact float node offsets), the centre
