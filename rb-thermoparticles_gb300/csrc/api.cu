@@ -141,9 +141,12 @@ int plane_sums(rbtp_handle *h)
     const bool parts = h->pb.np > 0;
     CK(launch_plane_sums(h->geo, h->ph, h->ux, h->uy, h->uz, h->phi, parts ? h->owner[h->ocur] : nullptr,
                          h->pb.state, h->pb.np, h->partials, h->nchunks, h->plane, h->stream));
-    h->plane_host.resize((size_t)NPLANEQ * h->geo.lx);
-    CK(cudaMemcpyAsync(h->plane_host.data(), h->plane, h->plane_host.size() * sizeof(double),
-                       cudaMemcpyDeviceToHost, h->stream));
+    const size_t n = (size_t)NPLANEQ * h->geo.lx;
+    if (!h->plane_host) {
+        h->plane_far.resize(n);
+        h->plane_host = h->plane_far.data();
+    }
+    CK(cudaMemcpyAsync(h->plane_host, h->plane, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     h->plane_valid = true;
     return RBTP_OK;
@@ -421,7 +424,12 @@ int rbtp_create(const rbtp_config *cfg, rbtp_handle **out)
     CKC(cudaMemsetAsync(h->ked, 0, L * sizeof(double), h->stream));
     CKC(dalloc(&h->status, 1));
     CKC(cudaMemsetAsync(h->status, 0, sizeof(DevStatus), h->stream));
-    CKC(cudaMallocHost(reinterpret_cast<void **>(&h->status_host), sizeof(DevStatus)));
+    // page-locked landing place of the status word and, behind it, of the plane sums (their copy does not go
+    // through a staging buffer); very long lattices keep the plane sums in ordinary memory
+    const size_t plane_bytes = cfg->lx <= 65536 ? (size_t)NPLANEQ * cfg->lx * sizeof(double) : 0;
+    CKC(cudaMallocHost(reinterpret_cast<void **>(&h->status_host), sizeof(DevStatus) + plane_bytes));
+    static_assert(sizeof(DevStatus) % sizeof(double) == 0, "the plane sums follow the status word");
+    if (plane_bytes) h->plane_host = reinterpret_cast<double *>(h->status_host + 1);
     const long long rows = (long long)cfg->ly * cfg->lz;
     h->nchunks = (int)std::min<long long>(rows, 512);
     CKC(dalloc(&h->partials, (size_t)h->nchunks * NPLANEQ * cfg->lx));
@@ -860,7 +868,7 @@ int rbtp_nu(rbtp_handle *h, int istep, rbtp_nu_row *row)
     if (!h->macros_valid) return fail(h, RBTP_ERR_STATE, "macroscopic fields were not materialised on the last step");
     s = plane_sums(h);
     if (s) return s;
-    return nu_from_planes(h, h->plane_host.data(), istep, row);
+    return nu_from_planes(h, h->plane_host, istep, row);
 }
 
 }  // extern "C"
@@ -914,7 +922,7 @@ int rbtp_means(rbtp_handle *h, double means[4])
     s = plane_sums(h);
     if (s) return s;
     const int lx = h->geo.lx;
-    const double *pl = h->plane_host.data();
+    const double *pl = h->plane_host;
     for (int k = 0; k < 4; ++k) {
         double a = 0.0;
         for (int ix = 0; ix < lx; ++ix) a += pl[(6 + k) * lx + ix];
@@ -935,7 +943,7 @@ int rbtp_profile(rbtp_handle *h, double *out)
     s = plane_sums(h);
     if (s) return s;
     const int lx = h->geo.lx;
-    const double *pl = h->plane_host.data();
+    const double *pl = h->plane_host;
     const double cnt = (double)h->geo.ly * (double)h->geo.lz;
     const double inv = cnt > 0 ? 1.0 / cnt : 0.0;
     for (int ix = 0; ix < lx; ++ix)

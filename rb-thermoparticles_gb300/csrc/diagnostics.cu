@@ -20,47 +20,68 @@ namespace {
 
 constexpr int PLANE_TX = 128;
 
-// Sums of plane ix over row chunk `chunk` of nchunks (rows = (y, z) pairs in z-major order).
+// Sums of plane ix over row chunk `chunk` of nchunks (rows = (y, z) pairs in z-major order), in row order.
+// The rows are loaded PLANE_ROWS at a time ahead of their sums, node counts are integers, and
+// the row's (y, z) is carried along (a 64-bit division per row and one row in flight took 620 us
+// at 320x320x160 instead of the 90 us that memory needs; the FP64 additions take 140).
+constexpr int PLANE_ROWS = 4;
 __device__ __forceinline__ void plane_partial_body(const Geo &geo, const Phys &ph, const double *ux,
                                                    const double *uy, const double *uz, const double *phi,
                                                    const int *owner, const double *pst, int np,
                                                    double *partials, int nchunks, int ix, int chunk)
 {
     const long long rows = (long long)geo.ly * geo.lz;
-    const long long r0 = rows * chunk / nchunks, r1 = rows * (chunk + 1) / nchunks;
+    const long long r0 = rows * chunk / nchunks;
+    const int nrows = (int)(rows * (chunk + 1) / nchunks - r0);
     double q[NPLANEQ];
 #pragma unroll
     for (int k = 0; k < NPLANEQ; ++k) q[k] = 0.0;
-    for (long long r = r0; r < r1; ++r) {
-        const int iz = (int)(r / geo.ly);
-        const int iy = (int)(r - (long long)iz * geo.ly);
-        const long long idx = (long long)iz * geo.lxy + (long long)iy * geo.lx + ix;
-        const double u = ux[idx], v = uy[idx], w = uz[idx], T = phi[idx];
-        const int own = owner ? owner[idx] : -1;
-        if (own < 0) {
-            q[0] += u * T;
-            q[1] += 1.0;
-            if (ix == 0) { q[4] += (ph.thot - T) / 0.5; q[5] += 1.0; }
-            else if (ix == geo.lx - 1) { q[4] += (T - ph.tcold) / 0.5; q[5] += 1.0; }
-            q[6] += u; q[7] += v; q[8] += w; q[9] += T;
-        } else {
-            q[2] += u * T;
-            q[3] += 1.0;
-            if (own < np) {
-                const double relx = ((double)ix + 0.5) - pst[0 * (long long)np + own];
-                const double rely = ((double)iy + 0.5) - pst[1 * (long long)np + own];
-                const double relz = ((double)iz + 0.5) - pst[2 * (long long)np + own];
-                const double wx = pst[18 * (long long)np + own], wy = pst[19 * (long long)np + own],
-                             wz = pst[20 * (long long)np + own];
-                q[6] += pst[3 * (long long)np + own] + (relz * wy - rely * wz);
-                q[7] += pst[4 * (long long)np + own] + (relx * wz - relz * wx);
-                q[8] += pst[5 * (long long)np + own] + (rely * wx - relx * wy);
-                q[9] += pst[30 * (long long)np + own];
-            } else {
+    int nfluid = 0, nsolid = 0;
+    int iz = (int)(r0 / geo.ly), iy = (int)(r0 - (long long)iz * geo.ly);
+    const long long base = r0 * geo.lx + ix;   // rows of all planes follow one another
+    for (int r = 0; r < nrows; r += PLANE_ROWS) {
+        double us[PLANE_ROWS], vs[PLANE_ROWS], ws[PLANE_ROWS], Ts[PLANE_ROWS];
+        int owns[PLANE_ROWS];
+#pragma unroll
+        for (int k = 0; k < PLANE_ROWS; ++k) {
+            const long long idx = base + (long long)min(r + k, nrows - 1) * geo.lx;
+            us[k] = ux[idx]; vs[k] = uy[idx]; ws[k] = uz[idx]; Ts[k] = phi[idx];
+            owns[k] = owner ? owner[idx] : -1;
+        }
+#pragma unroll
+        for (int k = 0; k < PLANE_ROWS; ++k) {
+            if (r + k >= nrows) break;
+            const double u = us[k], v = vs[k], w = ws[k], T = Ts[k];
+            const int own = owns[k];
+            if (own < 0) {
+                q[0] += u * T;
+                ++nfluid;
+                if (ix == 0) q[4] += (ph.thot - T) / 0.5;
+                else if (ix == geo.lx - 1) q[4] += (T - ph.tcold) / 0.5;
                 q[6] += u; q[7] += v; q[8] += w; q[9] += T;
+            } else {
+                q[2] += u * T;
+                ++nsolid;
+                if (own < np) {
+                    const double relx = ((double)ix + 0.5) - pst[0 * (long long)np + own];
+                    const double rely = ((double)iy + 0.5) - pst[1 * (long long)np + own];
+                    const double relz = ((double)iz + 0.5) - pst[2 * (long long)np + own];
+                    const double wx = pst[18 * (long long)np + own], wy = pst[19 * (long long)np + own],
+                                 wz = pst[20 * (long long)np + own];
+                    q[6] += pst[3 * (long long)np + own] + (relz * wy - rely * wz);
+                    q[7] += pst[4 * (long long)np + own] + (relx * wz - relz * wx);
+                    q[8] += pst[5 * (long long)np + own] + (rely * wx - relx * wy);
+                    q[9] += pst[30 * (long long)np + own];
+                } else {
+                    q[6] += u; q[7] += v; q[8] += w; q[9] += T;
+                }
             }
+            if (++iy == geo.ly) { iy = 0; ++iz; }
         }
     }
+    q[1] = (double)nfluid;
+    q[3] = (double)nsolid;
+    q[5] = ix == 0 || ix == geo.lx - 1 ? (double)nfluid : 0.0;
 #pragma unroll
     for (int k = 0; k < NPLANEQ; ++k) partials[((long long)chunk * NPLANEQ + k) * geo.lx + ix] = q[k];
 }
@@ -76,33 +97,48 @@ __global__ void __launch_bounds__(PLANE_TX) k_plane_partial(const Geo geo, const
     plane_partial_body(geo, ph, ux, uy, uz, phi, owner, pst, np, partials, nchunks, ix, blockIdx.y);
 }
 
-// Chunks are combined in ascending order: the plane sums are deterministic and identical in the
-// single-cavity and the batched reductions.
-__device__ __forceinline__ double plane_final_body(const double *partials, int nchunks, int lx, int t)
+// Sum of output t over the chunks, deterministic and the same in the single-cavity and the batched
+// reductions: FINAL_PARTS threads each add a contiguous part of the chunks in ascending order, and the
+// parts' sums are added in order (512 chunks in one chain of additions took 68 us).  Called by all
+// threads of a (FINAL_OUTS, FINAL_PARTS) block; the result is valid in the threads with y = 0.
+constexpr int FINAL_OUTS = 32, FINAL_PARTS = 16;
+__device__ __forceinline__ double plane_final_body(const double *partials, int nchunks, int lx, int t,
+                                                   double (&sh)[FINAL_PARTS][FINAL_OUTS])
 {
-    const int k = t / lx, ix = t - k * lx;
+    const int part = threadIdx.y, c0 = nchunks * part / FINAL_PARTS, c1 = nchunks * (part + 1) / FINAL_PARTS;
     double s = 0.0;
-    for (int c = 0; c < nchunks; ++c) s += partials[((long long)c * NPLANEQ + k) * lx + ix];
+    if (t < NPLANEQ * lx) {
+#pragma unroll 4
+        for (int c = c0; c < c1; ++c) s += partials[(long long)c * NPLANEQ * lx + t];
+    }
+    sh[part][threadIdx.x] = s;
+    __syncthreads();
+    if (part == 0)
+        for (int k = 1; k < FINAL_PARTS; ++k) s += sh[k][threadIdx.x];
+    __syncthreads();
     return s;
 }
 
-__global__ void k_plane_final(const Geo geo, const double *partials, int nchunks, double *plane)
+__global__ void __launch_bounds__(FINAL_OUTS * FINAL_PARTS) k_plane_final(const Geo geo, const double *partials,
+                                                                          int nchunks, double *plane)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= NPLANEQ * geo.lx) return;
-    plane[t] = plane_final_body(partials, nchunks, geo.lx, t);
+    __shared__ double sh[FINAL_PARTS][FINAL_OUTS];
+    const int t = blockIdx.x * FINAL_OUTS + threadIdx.x;
+    const double s = plane_final_body(partials, nchunks, geo.lx, t, sh);
+    if (threadIdx.y == 0 && t < NPLANEQ * geo.lx) plane[t] = s;
 }
 
 // Batched sampling, after the step's advance: cavities with samp_now set reduce their current
 // macroscopic fields (owners of the new solid flags, particle state after the update) exactly as
-// the single-cavity reduction does, and the final pass writes (step, plane sums) into the next slot
-// of the cavity's sample ring and bumps its sample counter.
+// the single-cavity reduction does; the first pass also counts the sample, and the final pass writes
+// (step, plane sums) into its slot of the cavity's sample ring.
 __global__ void __launch_bounds__(PLANE_TX) k_batch_sample_partial(const CavDesc *desc)
 {
     pdl_wait();
     pdl_trigger();
     const CavDesc &d = desc[blockIdx.y];
     if (!d.samp_now) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) d.status->nsamp += 1;
     const int *owner = d.pb.np > 0 ? d.owner[d.ocur] : nullptr;
     for (int chunk = blockIdx.x; chunk < d.nchunks; chunk += gridDim.x)
         for (int ix = threadIdx.x; ix < d.geo.lx; ix += PLANE_TX)
@@ -110,20 +146,22 @@ __global__ void __launch_bounds__(PLANE_TX) k_batch_sample_partial(const CavDesc
                                d.nchunks, ix, chunk);
 }
 
-__global__ void k_batch_sample_final(const CavDesc *desc)
+__global__ void __launch_bounds__(FINAL_OUTS * FINAL_PARTS) k_batch_sample_final(const CavDesc *desc)
 {
     pdl_wait();
     pdl_trigger();
-    const CavDesc &d = desc[blockIdx.x];
+    __shared__ double sh[FINAL_PARTS][FINAL_OUTS];
+    const CavDesc &d = desc[blockIdx.y];
     if (!d.samp_now) return;
     const int lx = d.geo.lx;
-    const int slot = d.status->nsamp % d.samp_cap;
+    const int slot = (d.status->nsamp - 1) % d.samp_cap;
     double *dst = d.samp + (long long)slot * (1 + NPLANEQ * lx);
-    for (int t = threadIdx.x; t < NPLANEQ * lx; t += blockDim.x)
-        dst[1 + t] = plane_final_body(d.partials, d.nchunks, lx, t);
-    if (threadIdx.x == 0) dst[0] = (double)d.istep;
-    __syncthreads();
-    if (threadIdx.x == 0) d.status->nsamp += 1;
+    for (int t0 = blockIdx.x * FINAL_OUTS; t0 < NPLANEQ * lx; t0 += gridDim.x * FINAL_OUTS) {
+        const int t = t0 + threadIdx.x;
+        const double s = plane_final_body(d.partials, d.nchunks, lx, t, sh);
+        if (threadIdx.y == 0 && t < NPLANEQ * lx) dst[1 + t] = s;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0 && threadIdx.y == 0) dst[0] = (double)d.istep;
 }
 
 // compute_Ked (collision.cu:91-152) and compute_ted (collision.cu:154-198) on the FP64 copy of
@@ -188,7 +226,7 @@ cudaError_t launch_batch_sample(const CavDesc *desc, int n, cudaStream_t st)
     if (n <= 0) return cudaSuccess;
     cudaError_t e = pdl_launch(k_batch_sample_partial, dim3(64, n), dim3(PLANE_TX), st, desc);
     if (e != cudaSuccess) return e;
-    return pdl_launch(k_batch_sample_final, dim3(n), dim3(256), st, desc);
+    return pdl_launch(k_batch_sample_final, dim3(16, n), dim3(FINAL_OUTS, FINAL_PARTS), st, desc);
 }
 
 cudaError_t launch_plane_sums(const Geo &geo, const Phys &ph, const double *ux, const double *uy,
@@ -199,7 +237,7 @@ cudaError_t launch_plane_sums(const Geo &geo, const Phys &ph, const double *ux, 
     const dim3 grd((geo.lx + PLANE_TX - 1) / PLANE_TX, nchunks, 1);
     k_plane_partial<<<grd, PLANE_TX, 0, st>>>(geo, ph, ux, uy, uz, phi, owner, pstate, np, partials, nchunks);
     const int n = NPLANEQ * geo.lx;
-    k_plane_final<<<(n + 255) / 256, 256, 0, st>>>(geo, partials, nchunks, plane);
+    k_plane_final<<<(n + FINAL_OUTS - 1) / FINAL_OUTS, dim3(FINAL_OUTS, FINAL_PARTS), 0, st>>>(geo, partials, nchunks, plane);
     return cudaGetLastError();
 }
 

@@ -42,7 +42,8 @@ struct rbtp_handle {
     // diagnostics
     double *partials = nullptr, *plane = nullptr;
     int nchunks = 1;
-    std::vector<double> plane_host;
+    double *plane_host = nullptr;    // plane sums on the host: behind status_host, or plane_far
+    std::vector<double> plane_far;
     bool plane_valid = false;
     // bookkeeping
     int istep = 0;
