@@ -278,7 +278,7 @@ def batch_variant(torch, steps: int, warmup: int, n: int = 256) -> dict:
            "cavities": n, "nodes": st["nodes"], "spheres": st["total_particles"],
            "ms_per_step": st["last_step_ms"], "mlups": st["nodes"] / st["last_step_ms"] / 1e3,
            "step_ms_p50": float(np.percentile(lat, 50)), "step_ms_p99": float(np.percentile(lat, 99)),
-           "tile_shape": ["32x4", "64x2"][st["tile_shape"]], "persistent_grid": st["grid"],
+           "tile_shape": ["128 consecutive nodes", "64x2"][st["tile_shape"]], "persistent_grid": st["grid"],
            "cuda_graph": bool(st["graph"]), "setup_seconds": round(setup, 2),
            "steps_run": warmup + 16 + steps + min(steps, 50) + 1,
            "members_nonfinite_at_end": nonfinite, "batch_calls_reporting_nonfinite": len(failed_calls)}

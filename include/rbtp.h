@@ -228,7 +228,7 @@ int  rbtp_checkpoint_read(rbtp_handle *h, const char *path);
  * NNUOUT, NFLOWOUT, NEND cadence and on its sampling cadence. */
 typedef struct rbtp_batch rbtp_batch;
 typedef struct rbtp_batch_stats {
-    int members, tiles, total_particles, tile_shape;   /* tile_shape: 0 = 32x4, 1 = 64x2 */
+    int members, tiles, total_particles, tile_shape;   /* tile_shape: 0 = 128 nodes, 1 = 64x2 */
     int grid, graph;                                    /* persistent blocks; 1 if replaying a graph */
     int tuned, reserved;
     double last_step_ms;                                /* device time of the last step (events) */

@@ -100,12 +100,13 @@ int rebuild(rbtp_batch *b)
 {
     drop_graph(b);
     const int n = (int)b->members.size();
-    const int tx[BATCH_SHAPES] = {32, 64}, ty[BATCH_SHAPES] = {4, 2};
+    const int tx[BATCH_SHAPES] = {128, 64}, ty[BATCH_SHAPES] = {1, 2};
     for (int s = 0; s < BATCH_SHAPES; ++s) {
         std::vector<int4> t;
         for (int m = 0; m < n; ++m) {
             const Geo &g = b->members[m]->geo;
-            const int nx = (g.lx + tx[s] - 1) / tx[s], ny = (g.ly + ty[s] - 1) / ty[s];
+            // ty = 1: runs of consecutive nodes of the plane, not of a row
+            const int nx = (int)(((ty[s] == 1 ? g.lxy : g.lx) + tx[s] - 1) / tx[s]), ny = ty[s] == 1 ? 1 : (g.ly + ty[s] - 1) / ty[s];
             for (int z = 0; z < g.lz; z += BATCH_TILE_Z)
                 for (int y = 0; y < ny; ++y)
                     for (int x = 0; x < nx; ++x) t.push_back(make_int4(m, x, y, z));

@@ -3,8 +3,8 @@
 // packed tile table, plus the small plan/advance kernels that keep each cavity's step state on the
 // device so that the whole step can be captured once in a CUDA graph and replayed.
 //
-// Tile table: int4 (cavity, tile_x, tile_y, z) for every TX x TY tile of every cavity, packed
-// cavity after cavity.  The persistent grid (chosen by the host autotuner, a multiple of the SM
+// Tile table: int4 (cavity, tile_x, tile_y, z) for every TX x TY tile of every cavity (TY = 1: runs of
+// TX consecutive nodes of the plane, tile_x-th), packed cavity after cavity.  The persistent grid (chosen by the host autotuner, a multiple of the SM
 // count) walks the table with a grid stride, so small and large cavities share the machine without
 // per-cavity launches.
 #include "step_node.cuh"
@@ -100,8 +100,20 @@ __global__ void __launch_bounds__(MODE == RBTP_STORE_F64 ? 2 * TX * TY : TX * TY
         }
         __syncthreads();
         // tile (member, x, y, z0): BATCH_TILE_Z planes from z0
-        const int ix = tl.y * TX + threadIdx.x, iy = tl.z * TY + threadIdx.y, z0 = tl.w;
-        const bool active = ix < sgeo.lx && iy < sgeo.ly;
+        const int z0 = tl.w;
+        int ix, iy;
+        bool active;
+        if constexpr (TY == 1) {
+            const unsigned n = (unsigned)tl.y * TX + threadIdx.x, lxy = (unsigned)sgeo.lxy;
+            active = n < lxy;
+            plane_node(sgeo, min(n, lxy - 1u), ix, iy);
+        } else {
+            ix = tl.y * TX + threadIdx.x;
+            iy = tl.z * TY + threadIdx.y;
+            active = ix < sgeo.lx && iy < sgeo.ly;
+            ix = min(ix, sgeo.lx - 1);
+            iy = min(iy, sgeo.ly - 1);
+        }
         if (d.out == OUT_IDLE || (!F64 && !active)) continue;
         StepBuffers b;
         b.f = d.f;
@@ -116,9 +128,8 @@ __global__ void __launch_bounds__(MODE == RBTP_STORE_F64 ? 2 * TX * TY : TX * TY
         for (int iz = z0; iz < z1; ++iz) {
             if constexpr (F64) {
                 extern __shared__ double smem64[];
-                const int cx = min(ix, sgeo.lx - 1), cy = min(iy, sgeo.ly - 1);
-                if (odd) step_node64<TX * TY, true, false>(sgeo, sph.kd, b, d.out, cx, cy, iz, active, smem64);
-                else step_node64<TX * TY, false, false>(sgeo, sph.kd, b, d.out, cx, cy, iz, active, smem64);
+                if (odd) step_node64<TX * TY, true, false>(sgeo, sph.kd, b, d.out, ix, iy, iz, active, smem64);
+                else step_node64<TX * TY, false, false>(sgeo, sph.kd, b, d.out, ix, iy, iz, active, smem64);
             } else {
                 if (odd) step_out<MODE, true>(sgeo, sph, soff, b, d.out, ix, iy, iz);
                 else step_out<MODE, false>(sgeo, sph, soff, b, d.out, ix, iy, iz);
@@ -135,7 +146,7 @@ cudaError_t launch_mode(int shape, const CavDesc *desc, const int4 *tiles, int n
     constexpr size_t smem = F64 ? step64_smem(128) : 0;
     constexpr int TZ = F64 ? 2 : 1;
     if (shape == 0)
-        return pdl_launch_dyn(k_step_batched<MODE, 32, 4>, dim3(grid), dim3(32, 4, TZ), smem, st, desc, tiles, ntiles);
+        return pdl_launch_dyn(k_step_batched<MODE, 128, 1>, dim3(grid), dim3(128, 1, TZ), smem, st, desc, tiles, ntiles);
     return pdl_launch_dyn(k_step_batched<MODE, 64, 2>, dim3(grid), dim3(64, 2, TZ), smem, st, desc, tiles, ntiles);
 }
 
@@ -144,7 +155,7 @@ cudaError_t launch_mode(int shape, const CavDesc *desc, const int4 *tiles, int n
 cudaError_t prepare_step_batched(int mode)
 {
     if (mode != RBTP_STORE_F64) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(k_step_batched<RBTP_STORE_F64, 32, 4>,
+    const cudaError_t e = cudaFuncSetAttribute(k_step_batched<RBTP_STORE_F64, 128, 1>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)step64_smem(128));
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(k_step_batched<RBTP_STORE_F64, 64, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(128, RBTP_STEP_MINB)
     step_node<MODE, ODD, OUT>(geo, ph, b, ao, ix, iy, iz);
 }
 
-// Block (32, 1, 2): 32 nodes of a row, f and g (step_node64.cuh).
+// Block (32, 1, 2): 32 consecutive nodes of a plane, f and g (step_node64.cuh).
 constexpr int NODES64 = 32;
 template <bool ODD, int OUT>
 __global__ void __launch_bounds__(2 * NODES64, step64_blocks(NODES64))
@@ -49,10 +49,10 @@ __global__ void __launch_bounds__(2 * NODES64, step64_blocks(NODES64))
     extern __shared__ double smem64[];
     pdl_wait();
     pdl_trigger();
-    const unsigned nx = (geo.lx + NODES64 - 1) / NODES64, iy = blockIdx.x / nx;
-    const int ix = (blockIdx.x - iy * nx) * NODES64 + threadIdx.x;
-    step_node64<NODES64, ODD, OUT == OUT_MACROS_COL>(geo, ph.kd, b, OUT, min(ix, geo.lx - 1), iy, blockIdx.y,
-                                                     ix < geo.lx, smem64);
+    const unsigned n = blockIdx.x * NODES64 + threadIdx.x, lxy = (unsigned)geo.lxy;
+    int ix, iy;
+    plane_node(geo, min(n, lxy - 1u), ix, iy);
+    step_node64<NODES64, ODD, OUT == OUT_MACROS_COL>(geo, ph.kd, b, OUT, ix, iy, blockIdx.y, n < lxy, smem64);
 }
 
 // Stream-only export: the post-streaming populations f(n) of the reference (its d_f / d_g after a
@@ -282,7 +282,7 @@ cudaError_t launch_step_mode(bool odd, int out, const Geo &geo, const Phys &ph,
     // and scatter (0.683 against 0.695 ms for 32-wide rows at 320x320x160); its even steps, which
     // touch no neighbour, run best in 64-node rows (0.583 against 0.596 ms for 32-wide rows).
     if constexpr (MODE == RBTP_STORE_F64) {
-        const dim3 grd((unsigned)((geo.lx + NODES64 - 1) / NODES64) * (unsigned)geo.ly, geo.lz);
+        const dim3 grd((unsigned)((geo.lxy + NODES64 - 1) / NODES64), geo.lz);
 #define RBTP_STEP_CASE(P, O)                                                                                     \
     if (odd == P && out == O)                                                                                    \
         return pdl_launch_dyn(k_step64<P, O>, grd, dim3(NODES64, 1, 2), step64_smem(NODES64), st, geo, ph, b);

@@ -209,6 +209,14 @@ struct Geo {
     long long lxy, L;
 };
 
+// (ix, iy) of node n of a z plane, rows one after another.
+__host__ __device__ __forceinline__ void plane_node(const Geo &geo, unsigned n, int &ix, int &iy)
+{
+    const unsigned y = n / (unsigned)geo.lx;
+    iy = (int)y;
+    ix = (int)(n - y * (unsigned)geo.lx);
+}
+
 // Slot offsets of the odd (swapped -> natural) step relative to a node's own slot of direction 0,
 // in elements: the gather of direction i reads slot (opp i, x - c_i) at g[i] = opp(i) L - off_i,
 // and the scatter of direction i writes slot (i, x + c_i) at i L + off_i = g[opp i]
@@ -460,7 +468,9 @@ struct CavDesc {
     double *partials;
 };
 
-constexpr int BATCH_SHAPES = 2;  // tile shapes of the batched step: 0 = 32x4, 1 = 64x2
+// tiles of the batched step: 0 = 128 consecutive nodes of a plane (no thread is left over at the rows'
+// ends: members of LX 32..96 in 32-wide tiles left a fifth of them idle), 1 = 64x2
+constexpr int BATCH_SHAPES = 2;
 // z-planes per tile of the batched step: a block stages its member's constants once and steps
 // BATCH_TILE_Z planes of its (x, y) tile
 #ifndef RBTP_BATCH_TILE_Z
