@@ -17,6 +17,11 @@ __host__ __device__ constexpr int place_dir(int p)
         if (dcx(i) == place_cx(p) && dcy(i) == place_cy(p) && dcz(i) == place_cz(p)) return i;
     return -1;
 }
+// direction index of (cx, cy, cz)
+__host__ __device__ constexpr int dir_at(int cx, int cy, int cz)
+{
+    return place_dir(9 * (cy + 1) + 3 * (cx + 1) + cz + 1);
+}
 // number of nonzero components of (cx, cz) at place q of a slab
 __host__ __device__ constexpr int slab_class(int q) { return (q / 3 != 1) + (q % 3 != 1); }
 
