@@ -112,7 +112,7 @@ __device__ __forceinline__ double *slot_at(double *base, unsigned i8, unsigned L
 // belong to two threads, which exchange the moments: six warps per scheduler.  The code loops over the
 // three slabs of directions: unrolled, its 75 KB did not stay in the instruction caches.  Measured
 // at 320x320x160: 4.4 ms per step, 13.1 ms with every sum on the FP64 pipe (424 FP64 instructions
-// per node there, 77 here; 880 B per node at the copy bandwidth would take 2.2 ms); at 64x64x32 46
+// per node there, 77 here; 880 B per node at the copy bandwidth would take 2.2 ms); at 64x64x32 43
 // against 118 us.  What bounds it now is the latency of the chain load - integer sums - FP64
 // coefficients - integer sums with the warps that fit (integer pipe 61 %, FP64 pipe 48 % busy).  `out`
 // selects the outputs (StepOut; COL: also the post-collision copies), `smem` is the block's shared
@@ -163,20 +163,41 @@ __device__ __forceinline__ void step_node64(const Geo &geo, const StepK<double> 
     }
     const double fold = is_g ? 0.0 : __ldg(static_cast<const double *>(b.faux) + node);
     copy_async_wait<0>();
-    // the populations g at places m become the Dirichlet image of the wall (streaming.cu:45-61): at the
-    // x walls a direction that leaves only through x takes the anti-bounce-back, y/z exits stay
-    // adiabatic
-    const bool image = ODD && is_g && out_x != 0u && active;
-    auto wall = [&](unsigned m, double density, auto &&put) {
-        const double tw = xlo ? K.thot : K.tcold;
+    // At the x walls a direction that leaves only through x takes the Dirichlet anti-bounce-back, y/z
+    // exits stay adiabatic (streaming.cu:45-61).  Few nodes of a warp lie there (two where rows are longer
+    // than 32), so the lanes share their images, one (node, direction) each: with every lane doing its
+    // own node's nine, an odd step of such a warp had 18 rounds with FP64 instructions (32x32x16: 11.4
+    // against 10.6 us per step, 64x64x32: 46.2 against 43.0, 320x320x160: 4.47 against 4.44 ms).
+    // `sign`: the populations that come from outside (-1) or leave (1) along their place's direction;
+    // put(the node's lane and index, place, image).
+    unsigned walls = 0u;
+    if constexpr (ODD) walls = is_g ? __ballot_sync(~0u, out_x != 0u && active) : 0u;
+    auto images = [&](int sign, auto &&density, auto &&put) {
+        const unsigned mine = (sign < 0 ? out_x & ~out_yz : __brev(out_x & ~out_yz) >> 5) | (xlo ? 1u << 27 : 0u);
+        const int lane = tn & 31, items = 9 * __popc(walls);
+        __syncwarp();
 #pragma unroll 1
-        for (; m; m &= m - 1) {
-            const int p = __ffs((int)m) - 1;
-            put(p, wall_image(pop[p * T], dweight_rt(c_place_dir8[p] / 8), tw, density));
+        for (int first = 0; first < items; first += 32) {
+            const int j = first + lane, k = j % 9;
+            unsigned rest = walls;
+#pragma unroll 1
+            for (int n = j / 9; n; --n) rest &= rest - 1;
+            const int at = j < items ? __ffs((int)rest) - 1 : lane;
+            const unsigned m = __shfl_sync(~0u, mine, at);
+            const bool lo = m >> 27;
+            const int p = k / 3 * 9 + k % 3 + (lo == (sign < 0) ? 6 : 0);
+            const double rho_w = density(at);
+            const int wall_node = __shfl_sync(~0u, (int)node, at);
+            if (j < items && (m >> p & 1u))
+                put(at, wall_node, p,
+                    wall_image(pop[p * T + at - lane], dweight_rt(c_place_dir8[p] / 8), lo ? K.thot : K.tcold, rho_w));
         }
+        __syncwarp();
     };
     // the even step's output, with the node's density of that step
-    if (image) wall(out_x & ~out_yz, b.rho_wall[wall_slot], [&](int p, double v) { pop[p * T] = v; });
+    if (walls)
+        images(-1, [&](int at) { return b.rho_wall[__shfl_sync(~0u, wall_slot, at)]; },
+               [&](int at, int, int p, double v) { pop[p * T + at - (tn & 31)] = v; });
 
     // ---- moments (macrovar.cu:3-34) and forcing, F_x = g0 beta (phi - T0) ----
     const Tops64 tops = tops64(pop, T);
@@ -249,7 +270,7 @@ __device__ __forceinline__ void step_node64(const Geo &geo, const StepK<double> 
             off = place_cx(q) + (s - 1) * lx + place_cz(q) * lxy;
         }
         *slot_at(N, i8, L, off) = r;
-        if (image) pop[p * T] = r;
+        if (ODD && is_g && out_x != 0u) pop[p * T] = r;
     };
     const double omega = is_g ? K.omc : K.om;
     if (!relax64(pop, T, omega, tops.weighted, c, [&](int s, const double(&r)[9]) {
@@ -266,9 +287,11 @@ __device__ __forceinline__ void step_node64(const Geo &geo, const StepK<double> 
     }
     // this step's output at the x walls, with this step's density: the population that left along p is
     // the next step's incoming one at 26 - p
-    if (image)
-        wall(__brev(out_x & ~out_yz) >> 5, rho,
-             [&](int p, double g) { *slot_at(N, c_place_dir8[26 - p], L, 0) = g; });
+    if (walls)
+        images(1, [&](int at) { return swap[RHO * NODES + at - (tn & 31)]; },
+               [&](int, int n, int p, double v) {
+                   *slot_at(static_cast<double *>(b.g) + n, c_place_dir8[26 - p], L, 0) = v;
+               });
 }
 
 }  // namespace rbtp
