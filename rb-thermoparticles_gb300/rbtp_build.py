@@ -31,7 +31,7 @@ NVCC_FLAGS = ARCH + [
     "-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr",
     "-Xcompiler", "-fPIC,-ffp-contract=off,-O2",
     "-I" + os.path.join(REPO, "include"),
-] + os.environ.get("XF","").split()
+]
 
 
 def nvcc() -> str:
@@ -78,7 +78,8 @@ def build(jobs: int = 0, host: bool = True, verbose: bool = False) -> str:
     _arch_guard()
     os.makedirs(LIBDIR, exist_ok=True)
     nv = nvcc()
-    headers = [os.path.join(CSRC, h) for h in ("rbtp_internal.cuh", "step_node.cuh", "handle.cuh", "fixed64.cuh", "collide64.cuh", "step_node64.cuh")]
+    headers = [os.path.join(CSRC, h) for h in ("rbtp_internal.cuh", "step_node.cuh", "handle.cuh", "fixed64.cuh",
+                                                "collide64.cuh", "step_node64.cuh")]
     headers.append(os.path.join(REPO, "include", "rbtp.h"))
     objs, todo = [], []
     for src in SOURCES:
