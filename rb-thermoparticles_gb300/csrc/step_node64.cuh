@@ -288,7 +288,7 @@ __device__ __forceinline__ void step_node64(const Geo &geo, const StepK<double> 
     // this step's output at the x walls, with this step's density: the population that left along p is
     // the next step's incoming one at 26 - p
     if (walls)
-        images(1, [&](int at) { return swap[RHO * NODES + at - (tn & 31)]; },
+        images(1, [&](int at) { return __shfl_sync(~0u, rho, at); },
                [&](int, int n, int p, double v) {
                    *slot_at(static_cast<double *>(b.g) + n, c_place_dir8[26 - p], L, 0) = v;
                });
