@@ -55,20 +55,27 @@ __global__ void k_batch_advance(CavDesc *desc, int n)
     }
 }
 
+// The batched kernel carries both parities of the step body behind block-uniform branches, in FP32 with
+// one body per output mode; it is given more registers than the single-cavity kernel (4 resident
+// blocks of 128) to keep them in registers (5 blocks: FP32 0.331 -> 0.358 ms, FP16s 0.250 -> 0.259).  Its
+// step body takes the scatter index from an opaque copy (FRESH_SCATTER), the odd-step offsets from the
+// member's AAOff staged in shared memory, and the face tests from per-node masks (FACE_MASK); see
+// step_node.cuh for what each is worth.  Shifted FP16, bound by instruction issue, takes the output
+// mode at run time, which leaves room in the instruction caches for the odd step's interior path: 32
+// members of 32 to 80 nodes across, per step 0.258 -> 0.250 ms without spheres, 0.402 -> 0.383 ms with
+// them.  FP32, bound by memory latency, ran 0.331 -> 0.341 ms with the same (0.338 without the
+// interior path).
 template <int MODE, bool ODD>
 __device__ __forceinline__ void step_out(const Geo &geo, const Phys &ph, const AAOff &ao, const StepBuffers &b,
                                          int out, int ix, int iy, int iz)
 {
-    if (out == OUT_NONE) step_node<MODE, ODD, OUT_NONE, false, true, true>(geo, ph, b, ao, ix, iy, iz);
+    if constexpr (MODE == RBTP_STORE_F16S)
+        step_node<MODE, ODD, OUT_RUNTIME, true, true, true>(geo, ph, b, ao, ix, iy, iz, out);
+    else if (out == OUT_NONE) step_node<MODE, ODD, OUT_NONE, false, true, true>(geo, ph, b, ao, ix, iy, iz);
     else if (out == OUT_RHO) step_node<MODE, ODD, OUT_RHO, false, true, true>(geo, ph, b, ao, ix, iy, iz);
     else step_node<MODE, ODD, OUT_MACROS, false, true, true>(geo, ph, b, ao, ix, iy, iz);
 }
 
-// The batched kernel carries all phase/output variants of the step body behind block-uniform
-// branches; it is given more registers than the single-cavity kernel (4 resident blocks of 128)
-// to keep them in registers.  Its step body takes the scatter index from an opaque copy
-// (FRESH_SCATTER), the odd-step offsets from the member's AAOff staged in shared memory, and the
-// face tests from per-node masks (FACE_MASK); see step_node.cuh for what each is worth.
 #ifndef RBTP_BATCH_MINB_LOW
 #define RBTP_BATCH_MINB_LOW 4
 #endif

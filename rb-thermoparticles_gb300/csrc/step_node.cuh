@@ -50,9 +50,11 @@ struct PairOps {
 // node's own slots only.  INTERIOR_PATH adds, for odd steps, a second copy of the gather and the
 // scatter without the box-face tests, taken by warps none of whose nodes touches a face.  It pays
 // only where the step is issue-bound (shifted-FP16 storage: odd step 0.683 against 0.84 ms without
-// it at 320x320x160); FP32 is HBM-bound (measured the same with it), and
-// the batched kernel (six step variants in one kernel at 128 registers) ran 0.7 % slower with it
-// (9,010 against 9,073 MLUPS for the 256-cavity ensemble), so they leave it out.
+// it at 320x320x160; batched see batch_step.cu); FP32 is HBM-bound (measured the same with it), and
+// the batched FP32 kernel ran 0.7 % slower with it (9,010 against 9,073 MLUPS for the 256-cavity
+// ensemble), so they leave it out.
+//
+// OUT: the outputs (StepOut), or OUT_RUNTIME with `out` (batched shifted FP16).
 //
 // FRESH_SCATTER: the scatter addresses its slots from an opaque copy of the node index.  A node
 // writes exactly the slots it read (both parities), so otherwise the compiler keeps the gather's
@@ -69,10 +71,11 @@ struct PairOps {
 // six face flags, instead of evaluating the flags' disjunction per direction.  Measured at
 // 320x320x160: batched ensemble +0.5 % (with the staged offset table); the single-cavity FP32 and shifted-FP16 odd steps run 1-2 % slower with it, so
 // they keep the flag expressions.
+constexpr int OUT_RUNTIME = -1;
 template <int MODE, bool ODD, int OUT, bool INTERIOR_PATH = MODE == RBTP_STORE_F16S, bool FRESH_SCATTER = false,
           bool FACE_MASK = false>
 __device__ __forceinline__ void step_node(const Geo &geo, const Phys &ph, const StepBuffers &b, const AAOff &ao,
-                                          int ix, int iy, int iz)
+                                          int ix, int iy, int iz, int out = OUT)
 {
     using ST = Store<MODE>;
     using S = typename ST::S;
@@ -267,13 +270,13 @@ __device__ __forceinline__ void step_node(const Geo &geo, const Phys &ph, const 
     const R Fx = K.g0b * (phi - K.t0);
     static_cast<A *>(b.faux)[node] = (A)Fx;
 
-    if constexpr (OUT >= OUT_MACROS) {
+    if (OUT == OUT_RUNTIME ? out >= OUT_MACROS : OUT >= OUT_MACROS) {
         b.rho[node] = (double)rho;
         b.ux[node] = (double)ux;
         b.uy[node] = (double)uy;
         b.uz[node] = (double)uz;
         b.phi[node] = (double)phi;
-    } else if constexpr (OUT == OUT_RHO) {
+    } else if (OUT == OUT_RUNTIME ? out == OUT_RHO : OUT == OUT_RHO) {
         b.rho[node] = (double)rho;
     }
     if constexpr (!ODD) {
