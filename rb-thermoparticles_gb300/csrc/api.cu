@@ -397,7 +397,6 @@ int rbtp_create(const rbtp_config *cfg, rbtp_handle **out)
             return cleanup_fail(e_ == cudaErrorMemoryAllocation ? RBTP_ERR_OOM : RBTP_ERR_CUDA); } \
     } while (0)
 
-    CKC(prepare_step(h->mode));
     CKC(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     {
         CKC(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));

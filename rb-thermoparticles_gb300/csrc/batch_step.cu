@@ -7,6 +7,8 @@
 // TX consecutive nodes of the plane, tile_x-th), packed cavity after cavity.  The persistent grid (chosen by the host autotuner, a multiple of the SM
 // count) walks the table with a grid stride, so small and large cavities share the machine without
 // per-cavity launches.
+#include <algorithm>
+
 #include "step_node.cuh"
 #include "step_node64.cuh"
 
@@ -76,13 +78,25 @@ __device__ __forceinline__ void step_out(const Geo &geo, const Phys &ph, const A
     else step_node<MODE, ODD, OUT_MACROS, false, true, true>(geo, ph, b, ao, ix, iy, iz);
 }
 
+__device__ __forceinline__ StepBuffers buffers(const CavDesc &d)
+{
+    StepBuffers b;
+    b.f = d.f;
+    b.g = d.g;
+    b.faux = d.faux;
+    b.rho_wall = d.rho_wall;
+    b.rho = d.rho; b.ux = d.ux; b.uy = d.uy; b.uz = d.uz; b.phi = d.phi;
+    b.fcol = nullptr; b.gcol = nullptr;
+    b.status = d.status;
+    return b;
+}
+
 #ifndef RBTP_BATCH_MINB_LOW
 #define RBTP_BATCH_MINB_LOW 4
 #endif
 
 template <int MODE, int TX, int TY>
-__global__ void __launch_bounds__(MODE == RBTP_STORE_F64 ? 2 * TX * TY : TX * TY,
-                                  MODE == RBTP_STORE_F64 ? step64_blocks(TX * TY) : RBTP_BATCH_MINB_LOW)
+__global__ void __launch_bounds__(TX * TY, RBTP_BATCH_MINB_LOW)
     k_step_batched(const CavDesc *__restrict__ desc, const int4 *__restrict__ tiles, int ntiles)
 {
     pdl_wait();
@@ -93,9 +107,8 @@ __global__ void __launch_bounds__(MODE == RBTP_STORE_F64 ? 2 * TX * TY : TX * TY
     __shared__ Phys sph;
     __shared__ AAOff soff;
     constexpr int GW = sizeof(Geo) / 4, PW = sizeof(Phys) / 4, OW = sizeof(AAOff) / 4;
-    constexpr bool F64 = MODE == RBTP_STORE_F64;   // two threads per node (step_node64.cuh)
-    constexpr int NT = F64 ? 2 * TX * TY : TX * TY;
-    const int tid = (threadIdx.z * TY + threadIdx.y) * TX + threadIdx.x;
+    constexpr int NT = TX * TY;
+    const int tid = threadIdx.y * TX + threadIdx.x;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int4 tl = tiles[t];
         const CavDesc &d = desc[tl.x];
@@ -121,26 +134,61 @@ __global__ void __launch_bounds__(MODE == RBTP_STORE_F64 ? 2 * TX * TY : TX * TY
             ix = min(ix, sgeo.lx - 1);
             iy = min(iy, sgeo.ly - 1);
         }
-        if (d.out == OUT_IDLE || (!F64 && !active)) continue;
-        StepBuffers b;
-        b.f = d.f;
-        b.g = d.g;
-        b.faux = d.faux;
-        b.rho_wall = d.rho_wall;
-        b.rho = d.rho; b.ux = d.ux; b.uy = d.uy; b.uz = d.uz; b.phi = d.phi;
-        b.fcol = nullptr; b.gcol = nullptr;
-        b.status = d.status;
+        if (d.out == OUT_IDLE || !active) continue;
+        const StepBuffers b = buffers(d);
         const int z1 = min(z0 + BATCH_TILE_Z, sgeo.lz);
         const bool odd = d.phase == PHASE_SWAPPED;
         for (int iz = z0; iz < z1; ++iz) {
-            if constexpr (F64) {
-                extern __shared__ double smem64[];
-                if (odd) step_node64<TX * TY, true, false>(sgeo, sph.kd, b, d.out, ix, iy, iz, active, smem64);
-                else step_node64<TX * TY, false, false>(sgeo, sph.kd, b, d.out, ix, iy, iz, active, smem64);
-            } else {
-                if (odd) step_out<MODE, true>(sgeo, sph, soff, b, d.out, ix, iy, iz);
-                else step_out<MODE, false>(sgeo, sph, soff, b, d.out, ix, iy, iz);
-            }
+            if (odd) step_out<MODE, true>(sgeo, sph, soff, b, d.out, ix, iy, iz);
+            else step_out<MODE, false>(sgeo, sph, soff, b, d.out, ix, iy, iz);
+        }
+    }
+}
+
+// FP64: the tiles in parts of 32 consecutive nodes, one warp pair each.
+template <int TX, int TY>
+__global__ void __launch_bounds__(2 * STEP64_NODES, STEP64_BLOCKS)
+    k_step64_batched(const CavDesc *__restrict__ desc, const int4 *__restrict__ tiles, int ntiles)
+{
+    pdl_wait();
+    pdl_trigger();
+    __shared__ double smem[STEP64_DOUBLES];
+    __shared__ Geo sgeo;
+    __shared__ StepK<double> sk;
+    constexpr int GW = sizeof(Geo) / 4, KW = sizeof(StepK<double>) / 4, PARTS = TX * TY / STEP64_NODES;
+    const int tid = threadIdx.z * STEP64_NODES + threadIdx.x;
+    for (int t = blockIdx.x; t < ntiles * PARTS; t += gridDim.x) {
+        const int4 tl = tiles[t / PARTS];
+        const int part = t % PARTS * STEP64_NODES;
+        const CavDesc &d = desc[tl.x];
+        if (d.out == OUT_IDLE) continue;
+        __syncthreads();   // the previous tile's readers are done
+        for (int k = tid; k < GW + KW; k += 2 * STEP64_NODES) {
+            if (k < GW) reinterpret_cast<int *>(&sgeo)[k] = reinterpret_cast<const int *>(&d.geo)[k];
+            else reinterpret_cast<int *>(&sk)[k - GW] = reinterpret_cast<const int *>(&d.ph.kd)[k - GW];
+        }
+        __syncthreads();
+        int ix, iy;
+        bool active;
+        if constexpr (TY == 1) {
+            const unsigned n0 = (unsigned)tl.y * TX + part, n = n0 + threadIdx.x, lxy = (unsigned)sgeo.lxy;
+            if (n0 >= lxy) continue;
+            active = n < lxy;
+            plane_node(sgeo, min(n, lxy - 1u), ix, iy);
+        } else {
+            const int x0 = tl.y * TX + part % TX;
+            iy = tl.z * TY + part / TX;
+            if (x0 >= sgeo.lx || iy >= sgeo.ly) continue;
+            ix = x0 + threadIdx.x;
+            active = ix < sgeo.lx;
+            ix = min(ix, sgeo.lx - 1);
+        }
+        const StepBuffers b = buffers(d);
+        const int z1 = min(tl.w + BATCH_TILE_Z, sgeo.lz);
+        const bool odd = d.phase == PHASE_SWAPPED;
+        for (int iz = tl.w; iz < z1; ++iz) {
+            if (odd) step_node64<true, false>(sgeo, sk, b, d.out, ix, iy, iz, active, smem);
+            else step_node64<false, false>(sgeo, sk, b, d.out, ix, iy, iz, active, smem);
         }
     }
 }
@@ -149,25 +197,18 @@ template <int MODE>
 cudaError_t launch_mode(int shape, const CavDesc *desc, const int4 *tiles, int ntiles, int grid, cudaStream_t st)
 {
     if (ntiles <= 0) return cudaSuccess;
-    constexpr bool F64 = MODE == RBTP_STORE_F64;
-    constexpr size_t smem = F64 ? step64_smem(128) : 0;
-    constexpr int TZ = F64 ? 2 : 1;
-    if (shape == 0)
-        return pdl_launch_dyn(k_step_batched<MODE, 128, 1>, dim3(grid), dim3(128, 1, TZ), smem, st, desc, tiles, ntiles);
-    return pdl_launch_dyn(k_step_batched<MODE, 64, 2>, dim3(grid), dim3(64, 2, TZ), smem, st, desc, tiles, ntiles);
+    if constexpr (MODE == RBTP_STORE_F64) {
+        // as many blocks more as a tile has parts
+        const dim3 g((unsigned)(std::min(grid, ntiles) * (128 / STEP64_NODES))), blk(STEP64_NODES, 1, 2);
+        if (shape == 0) return pdl_launch(k_step64_batched<128, 1>, g, blk, st, desc, tiles, ntiles);
+        return pdl_launch(k_step64_batched<64, 2>, g, blk, st, desc, tiles, ntiles);
+    } else {
+        if (shape == 0) return pdl_launch(k_step_batched<MODE, 128, 1>, dim3(grid), dim3(128, 1), st, desc, tiles, ntiles);
+        return pdl_launch(k_step_batched<MODE, 64, 2>, dim3(grid), dim3(64, 2), st, desc, tiles, ntiles);
+    }
 }
 
 }  // namespace
-
-cudaError_t prepare_step_batched(int mode)
-{
-    if (mode != RBTP_STORE_F64) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(k_step_batched<RBTP_STORE_F64, 128, 1>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)step64_smem(128));
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_step_batched<RBTP_STORE_F64, 64, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)step64_smem(128));
-}
 
 cudaError_t launch_batch_plan(CavDesc *desc, int n, cudaStream_t st)
 {

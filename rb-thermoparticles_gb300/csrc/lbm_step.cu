@@ -40,19 +40,18 @@ __global__ void __launch_bounds__(128, RBTP_STEP_MINB)
     step_node<MODE, ODD, OUT>(geo, ph, b, ao, ix, iy, iz);
 }
 
-// Block (32, 1, 2): 32 consecutive nodes of a plane, f and g (step_node64.cuh).
-constexpr int NODES64 = 32;
+// Blocks of 32 consecutive nodes of a plane, f and g (step_node64.cuh).
 template <bool ODD, int OUT>
-__global__ void __launch_bounds__(2 * NODES64, step64_blocks(NODES64))
+__global__ void __launch_bounds__(2 * STEP64_NODES, STEP64_BLOCKS)
     k_step64(const Geo geo, const Phys ph, const StepBuffers b)
 {
-    extern __shared__ double smem64[];
+    __shared__ double smem[STEP64_DOUBLES];
     pdl_wait();
     pdl_trigger();
-    const unsigned n = blockIdx.x * NODES64 + threadIdx.x, lxy = (unsigned)geo.lxy;
+    const unsigned n = blockIdx.x * STEP64_NODES + threadIdx.x, lxy = (unsigned)geo.lxy;
     int ix, iy;
     plane_node(geo, min(n, lxy - 1u), ix, iy);
-    step_node64<NODES64, ODD, OUT == OUT_MACROS_COL>(geo, ph.kd, b, OUT, ix, iy, blockIdx.y, n < lxy, smem64);
+    step_node64<ODD, OUT == OUT_MACROS_COL>(geo, ph.kd, b, OUT, ix, iy, blockIdx.y, n < lxy, smem);
 }
 
 // Stream-only export: the post-streaming populations f(n) of the reference (its d_f / d_g after a
@@ -282,10 +281,10 @@ cudaError_t launch_step_mode(bool odd, int out, const Geo &geo, const Phys &ph,
     // and scatter (0.683 against 0.695 ms for 32-wide rows at 320x320x160); its even steps, which
     // touch no neighbour, run best in 64-node rows (0.583 against 0.596 ms for 32-wide rows).
     if constexpr (MODE == RBTP_STORE_F64) {
-        const dim3 grd((unsigned)((geo.lxy + NODES64 - 1) / NODES64), geo.lz);
+        const dim3 grd((unsigned)((geo.lxy + STEP64_NODES - 1) / STEP64_NODES), geo.lz);
 #define RBTP_STEP_CASE(P, O)                                                                                     \
     if (odd == P && out == O)                                                                                    \
-        return pdl_launch_dyn(k_step64<P, O>, grd, dim3(NODES64, 1, 2), step64_smem(NODES64), st, geo, ph, b);
+        return pdl_launch(k_step64<P, O>, grd, dim3(STEP64_NODES, 1, 2), st, geo, ph, b);
         RBTP_STEP_CASE(true, OUT_NONE)
         RBTP_STEP_CASE(true, OUT_RHO)
         RBTP_STEP_CASE(true, OUT_MACROS)
@@ -327,25 +326,6 @@ cudaError_t launch_step(int mode, bool odd, int out, const Geo &geo, const Phys 
     case RBTP_STORE_F16S: return launch_step_mode<RBTP_STORE_F16S>(odd, out, geo, ph, b, st);
     }
     return cudaErrorInvalidValue;
-}
-
-cudaError_t prepare_step(int mode)
-{
-    if (mode != RBTP_STORE_F64) return cudaSuccess;
-    cudaError_t e = cudaSuccess;
-    auto allow = [&](auto *kernel) {
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)step64_smem(NODES64));
-    };
-    allow(k_step64<true, OUT_NONE>);
-    allow(k_step64<true, OUT_RHO>);
-    allow(k_step64<true, OUT_MACROS>);
-    allow(k_step64<true, OUT_MACROS_COL>);
-    allow(k_step64<false, OUT_NONE>);
-    allow(k_step64<false, OUT_RHO>);
-    allow(k_step64<false, OUT_MACROS>);
-    allow(k_step64<false, OUT_MACROS_COL>);
-    return e;
 }
 
 #define RBTP_MODE_DISPATCH(mode, CALL)                                  \

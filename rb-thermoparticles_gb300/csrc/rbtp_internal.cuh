@@ -38,12 +38,12 @@ __device__ __forceinline__ void pdl_trigger()
 #endif
 }
 template <typename... KArgs, typename... Args>
-cudaError_t pdl_launch_dyn(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args)
+cudaError_t pdl_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = 0;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -51,11 +51,6 @@ cudaError_t pdl_launch_dyn(void (*kernel)(KArgs...), dim3 grid, dim3 block, size
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-template <typename... KArgs, typename... Args>
-cudaError_t pdl_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args)
-{
-    return pdl_launch_dyn(kernel, grid, block, 0, st, args...);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -338,9 +333,6 @@ struct StepBuffers {
 
 cudaError_t launch_step(int mode, bool odd, int out, const Geo &geo, const Phys &ph,
                         const StepBuffers &b, cudaStream_t st);
-// Once per handle or batch, on its device: lets the FP64 step kernels take their shared memory.
-cudaError_t prepare_step(int mode);
-cudaError_t prepare_step_batched(int mode);
 // Post-streaming populations f(n) (the reference's d_f / d_g after a step) from an array in
 // PHASE_SWAPPED, as FP64 home layout: the odd step's gather, walls included, without collision.
 cudaError_t launch_stream_export(int mode, const Geo &geo, const Phys &ph, const void *fin,

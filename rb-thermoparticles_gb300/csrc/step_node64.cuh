@@ -7,16 +7,16 @@
 
 namespace rbtp {
 
-// An FP64 step block: NODES nodes, two threads each, one for f (threadIdx.z = 0) and one for g, so that a
-// warp of f works beside its partner warp of g.  Shared memory: the 27 populations of thread t at
-// [place][t] (places of collide64.cuh), which no other thread touches, and what the two threads of a node
-// exchange.  The single-cavity step takes blocks of one warp pair (a block's shared memory is free
-// again when its slowest warp is done: 4.45 against 4.65 ms per step at 320x320x160 for four
-// pairs), the batched one the 128 nodes of its tiles.
-constexpr int STEP64_SWAP = 16;   // doubles exchanged per node
-constexpr size_t step64_smem(int nodes) { return (size_t)(27 * 2 + STEP64_SWAP) * nodes * sizeof(double); }
-// resident blocks: 24 warps per SM, by registers (80 per thread) and shared memory (18 KB per warp pair)
-constexpr int step64_blocks(int nodes) { return 384 / nodes; }
+// An FP64 step block (32, 1, 2): 32 consecutive nodes of a row or plane, two threads each, one for f
+// (threadIdx.z = 0) and one for g, so that a warp of f works beside its partner warp of g.  Shared
+// memory: the 27 populations of thread t at [place][t] (places of collide64.cuh), and what the two
+// threads of a node exchange.  A block is one warp pair, whose shared memory is free again when its
+// slower warp is done (four pairs: 4.65 against 4.45 ms per step at 320x320x160, and 1.41 against
+// 1.35 ms for a batch of 32 members of 32 to 80 nodes across).
+constexpr int STEP64_NODES = 32;
+constexpr int STEP64_SWAP = 16;      // doubles exchanged per node
+constexpr int STEP64_DOUBLES = (27 * 2 + STEP64_SWAP) * STEP64_NODES;
+constexpr int STEP64_BLOCKS = 12;    // resident per SM, by registers (80 per thread) and shared memory (18 KB)
 
 // eight times the direction index of a place, for loops that are not unrolled, and dir_mask by places
 static __constant__ int c_place_dir8[27] = {200, 72, 168, 144, 32, 112, 208, 80, 176, 136, 24, 104, 48, 0, 40, 120, 8, 88, 192, 64, 160, 128, 16, 96, 184, 56, 152};
@@ -39,24 +39,6 @@ template <int LEFT>
 __device__ __forceinline__ void copy_async_wait()
 {
     asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
-}
-
-// The barrier of a warp of f with its partner of g.  Its number is a constant in each case: with a
-// number from a register the compiler reserves all 16 barriers for the block, and an SM has only 64.
-template <int NODES>
-__device__ __forceinline__ void partner_sync()
-{
-    if constexpr (NODES == 32) {
-        asm volatile("bar.sync 1, 64;" ::: "memory");
-    } else {
-        static_assert(NODES == 128, "one barrier per warp pair");
-        switch ((threadIdx.y * blockDim.x + threadIdx.x) / 32) {
-        case 0: asm volatile("bar.sync 1, 64;" ::: "memory"); break;
-        case 1: asm volatile("bar.sync 2, 64;" ::: "memory"); break;
-        case 2: asm volatile("bar.sync 3, 64;" ::: "memory"); break;
-        default: asm volatile("bar.sync 4, 64;" ::: "memory"); break;
-        }
-    }
 }
 
 // Moments and collision in plain FP64 operations for the values that the grids do not take (beyond
@@ -118,11 +100,11 @@ __device__ __forceinline__ double *slot_at(double *base, unsigned i8, unsigned L
 // selects the outputs (StepOut; COL: also the post-collision copies), `smem` is the block's shared
 // memory.  Threads that are not `active` only take part in the barriers; they read the slots of the
 // node they are given (which must exist).
-template <int NODES, bool ODD, bool COL>
+template <bool ODD, bool COL>
 __device__ __forceinline__ void step_node64(const Geo &geo, const StepK<double> &K, const StepBuffers &b, int out,
                                             int ix, int iy, int iz, bool active, double *smem)
 {
-    constexpr int T = 2 * NODES;
+    constexpr int NODES = STEP64_NODES, T = 2 * NODES;
     const bool is_g = threadIdx.z != 0;
     const int tn = threadIdx.y * blockDim.x + threadIdx.x;
     double *const pop = smem + (is_g ? NODES : 0) + tn;
@@ -220,7 +202,7 @@ __device__ __forceinline__ void step_node64(const Geo &geo, const StepK<double> 
         swap[UY * NODES] = my;
         swap[UZ * NODES] = mz;
     }
-    partner_sync<NODES>();
+    __syncthreads();
     const double rho = swap[RHO * NODES], ux = swap[UX * NODES], Fx = swap[FX * NODES];
     if (active) {
         if (is_g) static_cast<double *>(b.faux)[node] = Fx;
@@ -243,7 +225,7 @@ __device__ __forceinline__ void step_node64(const Geo &geo, const StepK<double> 
     Vel64 v;
     if (is_g) {
         const Src64 src = src64(rho, ux, swap[UY * NODES], swap[UZ * NODES], m0, Fx, mx, my, mz, K);
-        partner_sync<NODES>();
+        __syncthreads();
         double *const vv = &v.x;
 #pragma unroll
         for (int k = 0; k < 10; ++k) vv[k] = swap[(VEL + k) * NODES];
@@ -253,7 +235,7 @@ __device__ __forceinline__ void step_node64(const Geo &geo, const StepK<double> 
         const double *const vv = &v.x;
 #pragma unroll
         for (int k = 0; k < 10; ++k) swap[(VEL + k) * NODES] = vv[k];
-        partner_sync<NODES>();
+        __syncthreads();
         coef64_f(c, rho, ux, Fx, v, K);
     }
 
