@@ -109,9 +109,9 @@ cudaError_t aux_from_host(rbtp_handle *h, const double *src)
 
 // Build the current solid flags and the IBB link slabs from the current particle positions
 // (build_links, links.cu:143-256).
-int build_links(rbtp_handle *h, int *owner, bool pgeo_fresh = false)
+int build_links(rbtp_handle *h, int *owner)
 {
-    CK(launch_mark(h->geo, h->ph, h->pb, owner, h->stream, !pgeo_fresh));
+    CK(launch_mark(h->geo, h->ph, h->pb, owner, h->stream));
     CK(launch_link_fill(h->mode, h->geo, h->ph, h->pb, owner, h->status, h->stream));
     return RBTP_OK;
 }
@@ -660,14 +660,17 @@ int rbtp_step_ex(rbtp_handle *h, int nsteps, unsigned flags)
         b.fcol = h->fcol; b.gcol = h->gcol; b.status = h->status;
         CK(launch_step(h->mode, odd, out, h->geo, h->ph, b, h->stream));
         if (parts) {
-            // Stream order: the contacts (positions only) run on the side stream beside IBB (both
-            // latency-bound, few CTAs); the integrator waits for the contact forces.  The link
-            // slabs stay on the main stream: beside the HBM-bound bulk kernel their CTAs would take
-            // its SM slots (measured slower).  The particle kernels use ordinary launches:
-            // programmatic dependent launch, which lets each one's blocks become resident while
-            // its predecessor finishes, made the 1000-sphere step 0.3 % (FP32) and 0.6 % (FP64)
-            // slower.
+            // Stream order: the contacts (positions only) run on the side stream beside IBB
+            // (latency-bound, few CTAs); the integrator waits for the contact forces.  The new link
+            // slabs, which the next step's IBB takes, are filled beside the refill (with the
+            // clears in one kernel: 64x64x32 with 9 spheres 103 -> 83 us per step in FP32 and
+            // 153 -> 128 in FP64, 1000 spheres in FP32 1.73 -> 1.71 ms), but not beside the next
+            // HBM-bound bulk kernel, whose SM slots their CTAs would take (measured slower).  The
+            // particle kernels use ordinary launches: programmatic dependent launch, which lets
+            // each one's blocks become resident while its predecessor finishes, made the
+            // 1000-sphere step 0.3 % (FP32) and 0.6 % (FP64) slower.
             int *oc = h->owner[h->ocur], *on = h->owner[1 - h->ocur];
+            CK(launch_step_clear(h->geo, h->pb, on, h->status, h->stream));
             CK(cudaEventRecord(h->ev_fork, h->stream));
             CK(cudaStreamWaitEvent(h->side, h->ev_fork, 0));
             CK(launch_contacts(h->geo, h->ph, h->pb, h->status, h->side));
@@ -675,10 +678,14 @@ int rbtp_step_ex(rbtp_handle *h, int nsteps, unsigned flags)
             CK(launch_links_ibb(h->mode, h->geo, h->ph, h->pb, h->f, h->g, h->rho, odd, h->stream));
             CK(cudaStreamWaitEvent(h->stream, h->ev_side, 0));
             CK(launch_update(h->geo, h->ph, h->pb, h->stream));   // also refreshes the geometry cache
-            s = build_links(h, on, true);
-            if (s) return s;
+            CK(launch_mark(h->geo, h->ph, h->pb, on, h->stream, false));
+            CK(cudaEventRecord(h->ev_fork, h->stream));
+            CK(cudaStreamWaitEvent(h->side, h->ev_fork, 0));
+            CK(launch_link_fill(h->mode, h->geo, h->ph, h->pb, on, h->status, h->side));
+            CK(cudaEventRecord(h->ev_side, h->side));
             CK(launch_refill(h->mode, h->geo, h->ph, h->pb, oc, on, h->f, h->g, h->faux, h->rho_wall, macro,
                              h->rho, h->ux, h->uy, h->uz, h->phi, h->status, odd, h->stream));
+            CK(cudaStreamWaitEvent(h->stream, h->ev_side, 0));
             h->ocur = 1 - h->ocur;
         }
         h->phase = odd ? PHASE_HOME : PHASE_SWAPPED;

@@ -1402,6 +1402,30 @@ __global__ void k_refill_scatter(const Geo geo, const Phys ph, const PartBuffers
 
 }  // namespace
 
+namespace {
+
+// What a step's particle kernels count or mark from zero: the contact cells, the contact and new-fluid
+// counters, and the solid flags of the positions to come, in one kernel instead of five memory sets.
+__device__ __forceinline__ void step_clear_body(const PartBuffers &pb, int *owner, long long L)
+{
+    const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+    const int cells = pb.ncell[0] * pb.ncell[1] * pb.ncell[2];
+    for (long long c = first; c < cells; c += stride) {
+        pb.cell_count[c] = 0;
+        pb.cell_fill[c] = 0;
+    }
+    for (long long i = first; i < L / 4; i += stride) reinterpret_cast<int4 *>(owner)[i] = make_int4(-1, -1, -1, -1);
+    if (first < L % 4) owner[L - 1 - first] = -1;
+}
+
+__global__ void k_step_clear(const Geo geo, const PartBuffers pb, int *owner, DevStatus *status)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0) status->ncontacts = status->nf_count = 0;
+    step_clear_body(pb, owner, geo.L);
+}
+
+}  // namespace
+
 #define RBTP_MODE_DISPATCH(mode, CALL)                                      \
     switch (mode) {                                                         \
     case RBTP_STORE_F64: { constexpr int M = RBTP_STORE_F64; CALL; break; }  \
@@ -1418,15 +1442,19 @@ cudaError_t launch_links_ibb(int mode, const Geo &geo, const Phys &ph, const Par
     return cudaGetLastError();
 }
 
+cudaError_t launch_step_clear(const Geo &geo, const PartBuffers &pb, int *owner, DevStatus *status, cudaStream_t st)
+{
+    if (pb.np <= 0) return cudaSuccess;
+    const int blocks = (int)std::min<long long>(608, (geo.L / 4 + 255) / 256 + 1);
+    k_step_clear<<<blocks, 256, 0, st>>>(geo, pb, owner, status);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_contacts(const Geo &geo, const Phys &ph, const PartBuffers &pb,
                             DevStatus *status, cudaStream_t st)
 {
     if (pb.np <= 0) return cudaSuccess;
     const int ncells = pb.ncell[0] * pb.ncell[1] * pb.ncell[2];
-    cudaError_t e;
-    if ((e = cudaMemsetAsync(pb.cell_count, 0, sizeof(int) * ncells, st))) return e;
-    if ((e = cudaMemsetAsync(pb.cell_fill, 0, sizeof(int) * ncells, st))) return e;
-    if ((e = cudaMemsetAsync(&status->ncontacts, 0, sizeof(int), st))) return e;
     const int t = 128, bl = (pb.np + t - 1) / t;
     k_cell_count<<<bl, t, 0, st>>>(pb);
     k_cell_scan<<<1, 1024, 0, st>>>(pb, ncells);
@@ -1443,12 +1471,14 @@ cudaError_t launch_update(const Geo &geo, const Phys &ph, const PartBuffers &pb,
 }
 
 cudaError_t launch_mark(const Geo &geo, const Phys &ph, const PartBuffers &pb, int *owner_out,
-                        cudaStream_t st, bool pgeo)
+                        cudaStream_t st, bool fresh)
 {
-    cudaError_t e = cudaMemsetAsync(owner_out, 0xFF, sizeof(int) * (size_t)geo.L, st);
-    if (e) return e;
+    if (fresh) {
+        const cudaError_t e = cudaMemsetAsync(owner_out, 0xFF, sizeof(int) * (size_t)geo.L, st);
+        if (e) return e;
+    }
     if (pb.np <= 0) return cudaSuccess;
-    if (pgeo) k_pgeo<<<(pb.np + UPDATE_WARPS - 1) / UPDATE_WARPS, 32 * UPDATE_WARPS, 0, st>>>(geo, ph, pb);
+    if (fresh) k_pgeo<<<(pb.np + UPDATE_WARPS - 1) / UPDATE_WARPS, 32 * UPDATE_WARPS, 0, st>>>(geo, ph, pb);
     if (pb.np < PARTICLES_WIDE) k_mark<LINK_WIDE><<<pb.np, LINK_WIDE, 0, st>>>(geo, ph, pb, owner_out);
     else k_mark<LINK_NARROW><<<pb.np, LINK_NARROW, 0, st>>>(geo, ph, pb, owner_out);
     return cudaGetLastError();
@@ -1476,8 +1506,6 @@ cudaError_t launch_refill(int mode, const Geo &geo, const Phys &ph, const PartBu
                           bool odd, cudaStream_t st)
 {
     if (pb.np <= 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(&status->nf_count, 0, sizeof(int), st);
-    if (e) return e;
     if (pb.np < PARTICLES_WIDE)
         k_new_fluid<LINK_WIDE><<<pb.np, LINK_WIDE, 0, st>>>(geo, ph, pb, owner_prev, owner_cur, status);
     else
@@ -1509,17 +1537,13 @@ __global__ void __launch_bounds__(IBB_THREADS, MODE == RBTP_STORE_F64 ? 4 : 6) k
     links_ibb_body<MODE>(d.geo, d.ph, d.pb, d.f, d.g, d.rho, d.phase == PHASE_SWAPPED, mp.y, cm.y, sh);
 }
 
-__global__ void k_cells_zero_b(const CavDesc *desc, const int *pmem)
+__global__ void k_step_clear_b(const CavDesc *desc, const int *pmem)
 {
     pdl_wait();
     pdl_trigger();
     const CavDesc &d = desc[pmem[blockIdx.y]];
     if (d.out == OUT_IDLE) return;
-    const int n = d.pb.ncell[0] * d.pb.ncell[1] * d.pb.ncell[2];
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-        d.pb.cell_count[c] = 0;
-        d.pb.cell_fill[c] = 0;
-    }
+    step_clear_body(d.pb, d.owner[d.ocur ^ 1], d.geo.L);
 }
 
 __global__ void k_cell_count_b(const CavDesc *desc, const int2 *pmap, int total)
@@ -1581,18 +1605,6 @@ __global__ void __launch_bounds__(32 * UPDATE_WARPS) k_update_b(const CavDesc *d
     const CavDesc &d = desc[mp.x];
     if (d.out == OUT_IDLE) return;
     update_warp(d.geo, d.ph, d.pb, mp.y);
-}
-
-__global__ void k_owner_fill_b(const CavDesc *desc, const int *pmem)
-{
-    pdl_wait();
-    pdl_trigger();
-    const CavDesc &d = desc[pmem[blockIdx.y]];
-    if (d.out == OUT_IDLE) return;
-    int *o = d.owner[d.ocur ^ 1];
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < d.geo.L;
-         i += (long long)gridDim.x * blockDim.x)
-        o[i] = -1;
 }
 
 template <int NT>
@@ -1670,10 +1682,10 @@ cudaError_t particles_batched_mode(const CavDesc *desc, const int2 *pmap, int to
     do {                                                                    \
         if ((e = pdl_launch(__VA_ARGS__)) != cudaSuccess) return e;         \
     } while (0)
-    // contacts (cell list and pair forces of the current positions) beside IBB
+    // beside IBB: the clears, then the contacts (cell list and pair forces of the current positions)
     if ((e = cudaEventRecord(ev_fork, st)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(side, ev_fork, 0)) != cudaSuccess) return e;
-    RBTP_PDL(k_cells_zero_b, dim3(4, npmem), dim3(256), side, desc, pmem);
+    RBTP_PDL(k_step_clear_b, dim3(64, npmem), dim3(256), side, desc, pmem);
     RBTP_PDL(k_cell_count_b, dim3(bl), dim3(t), side, desc, pmap, total);
     RBTP_PDL(k_cell_scan_b, dim3(npmem), dim3(1024), side, desc, pmem);
     RBTP_PDL(k_cell_fill_b, dim3(bl), dim3(t), side, desc, pmap, total);
@@ -1683,20 +1695,22 @@ cudaError_t particles_batched_mode(const CavDesc *desc, const int2 *pmap, int to
     RBTP_PDL(k_links_ibb_b<MODE>, dim3(ncmap), dim3(IBB_THREADS), st, desc, pmap, cmap);
     if ((e = cudaStreamWaitEvent(st, ev_join, 0)) != cudaSuccess) return e;
     RBTP_PDL(k_update_b, dim3((total + UPDATE_WARPS - 1) / UPDATE_WARPS), dim3(32 * UPDATE_WARPS), st, desc, pmap, total);
-    RBTP_PDL(k_owner_fill_b, dim3(64, npmem), dim3(256), st, desc, pmem);
-    if (total < PARTICLES_WIDE) {
-        RBTP_PDL(k_mark_b<LINK_WIDE>, dim3(total), dim3(LINK_WIDE), st, desc, pmap);
-        RBTP_PDL(k_link_fill_b<MODE != RBTP_STORE_F64, LINK_WIDE>, dim3(total), dim3(LINK_WIDE), st, desc, pmap);
-        RBTP_PDL(k_new_fluid_b<LINK_WIDE>, dim3(total), dim3(LINK_WIDE), st, desc, pmap);
-    } else {
-        RBTP_PDL(k_mark_b<LINK_NARROW>, dim3(total), dim3(LINK_NARROW), st, desc, pmap);
-        RBTP_PDL(k_link_fill_b<MODE != RBTP_STORE_F64, LINK_NARROW>, dim3(total), dim3(LINK_NARROW), st, desc, pmap);
-        RBTP_PDL(k_new_fluid_b<LINK_NARROW>, dim3(total), dim3(LINK_NARROW), st, desc, pmap);
-    }
+    const bool wide = total < PARTICLES_WIDE;
+    if (wide) RBTP_PDL(k_mark_b<LINK_WIDE>, dim3(total), dim3(LINK_WIDE), st, desc, pmap);
+    else RBTP_PDL(k_mark_b<LINK_NARROW>, dim3(total), dim3(LINK_NARROW), st, desc, pmap);
+    // the new links, which the next step's IBB takes, beside the refill
+    if ((e = cudaEventRecord(ev_fork, st)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(side, ev_fork, 0)) != cudaSuccess) return e;
+    constexpr bool F = MODE != RBTP_STORE_F64;
+    if (wide) RBTP_PDL(k_link_fill_b<F, LINK_WIDE>, dim3(total), dim3(LINK_WIDE), side, desc, pmap);
+    else RBTP_PDL(k_link_fill_b<F, LINK_NARROW>, dim3(total), dim3(LINK_NARROW), side, desc, pmap);
+    if ((e = cudaEventRecord(ev_join, side)) != cudaSuccess) return e;
+    if (wide) RBTP_PDL(k_new_fluid_b<LINK_WIDE>, dim3(total), dim3(LINK_WIDE), st, desc, pmap);
+    else RBTP_PDL(k_new_fluid_b<LINK_NARROW>, dim3(total), dim3(LINK_NARROW), st, desc, pmap);
     RBTP_PDL(k_refill_compute_b<MODE>, dim3(16, npmem), dim3(256), st, desc, pmem);
     RBTP_PDL(k_refill_scatter_b<MODE>, dim3(8, npmem), dim3(256), st, desc, pmem);
 #undef RBTP_PDL
-    return cudaGetLastError();
+    return cudaStreamWaitEvent(st, ev_join, 0);
 }
 
 }  // namespace

@@ -415,13 +415,16 @@ struct PartBuffers {
 // describes).
 cudaError_t launch_links_ibb(int mode, const Geo &geo, const Phys &ph, const PartBuffers &pb,
                              void *f, void *g, const double *rho, bool odd, cudaStream_t st);
+// What the step's contacts, marking (into owner) and new-fluid search start from.
+cudaError_t launch_step_clear(const Geo &geo, const PartBuffers &pb, int *owner, DevStatus *status, cudaStream_t st);
 cudaError_t launch_contacts(const Geo &geo, const Phys &ph, const PartBuffers &pb,
                             DevStatus *status, cudaStream_t st);
 // The integrator also refreshes the particles' geometry cache (PGeo) for their new positions.
 cudaError_t launch_update(const Geo &geo, const Phys &ph, const PartBuffers &pb, cudaStream_t st);
-// pgeo: refresh the geometry cache first (false right after launch_update, which did it)
+// fresh: clear the flags and refresh the geometry cache first (within a step launch_step_clear and
+// launch_update did)
 cudaError_t launch_mark(const Geo &geo, const Phys &ph, const PartBuffers &pb, int *owner_out,
-                        cudaStream_t st, bool pgeo = true);
+                        cudaStream_t st, bool fresh = true);
 cudaError_t launch_link_fill(int mode, const Geo &geo, const Phys &ph, const PartBuffers &pb,
                              const int *owner, DevStatus *status, cudaStream_t st);
 cudaError_t launch_refill(int mode, const Geo &geo, const Phys &ph, const PartBuffers &pb,
