@@ -729,9 +729,12 @@ constexpr int PARTICLES_WIDE = 4 * 152;
 
 constexpr int CONTACT_WARPS = 4;   // particles per 128-thread CTA, one warp each
 
-// One warp per particle: lane k < 27 scans neighbour cell k of the particle's cell, accepted
-// partners are collected in shared memory, and lane 0 sorts them and adds the pair forces in
-// ascending partner order (the order pforces.cu's pair loop adds them to p), then the walls.
+// One warp per particle: lane k < 27 scans neighbour cell k of the particle's cell, accepted partners
+// are collected in shared memory and sorted; a lane each computes their pair forces, which lane 0
+// adds up in ascending partner order (the order pforces.cu's pair loop adds them to p), then the
+// walls', computed by six lanes.  The kernel is a chain of FP64 operations (64 cycles each for the
+// warp, a square root or a division a thousand and more), so pairs that are certainly apart are
+// dismissed on the squared distance, and what lanes can do side by side they do.
 __device__ __forceinline__ void contact_force_body(const Geo &geo, const Phys &ph,
                                                    const PartBuffers &pb, DevStatus *status, int p,
                                                    int *cand /* MAX_CAND */, int &ncand)
@@ -744,6 +747,8 @@ __device__ __forceinline__ void contact_force_body(const Geo &geo, const Phys &p
     if (lane == 0) ncand = 0;
     __syncwarp();
     if (np > 1 && lane < 27) {
+        const double reach = 2.0 * radius + min_gap;
+        const double apart = reach > 0.0 ? reach * reach * (1.0 + 1e-9) : __longlong_as_double(0x7ff0000000000000LL);   // rounding is far below 1e-9
         const int cx = cell_of(x, pb.cell_size, pb.ncell[0]);
         const int cy = cell_of(y, pb.cell_size, pb.ncell[1]);
         const int cz = cell_of(z, pb.cell_size, pb.ncell[2]);
@@ -758,7 +763,7 @@ __device__ __forceinline__ void contact_force_body(const Geo &geo, const Phys &p
                 const double dy = dsub(y, PCOL(st, np, 1, q));
                 const double dz = dsub(z, PCOL(st, np, 2, q));
                 const double dsq = sq3(dx, dy, dz);
-                if (dsq <= 1.0e-12) continue;
+                if (dsq <= 1.0e-12 || dsq > apart) continue;
                 const double hgap = dsub(__dsqrt_rn(dsq), dmul(2.0, radius));
                 if (hgap >= min_gap) continue;
                 const int slot = atomicAdd(&ncand, 1);
@@ -767,61 +772,70 @@ __device__ __forceinline__ void contact_force_body(const Geo &geo, const Phys &p
         }
     }
     __syncwarp();
-    if (lane != 0) return;
     int nc = ncand;
-    if (nc > MAX_CAND) {
-        atomicOr(&status->contact_overflow, 1);
-        nc = MAX_CAND;
-    }
-    for (int i = 1; i < nc; ++i) {
-        const int v = cand[i];
-        int j = i - 1;
-        while (j >= 0 && cand[j] > v) { cand[j + 1] = cand[j]; --j; }
-        cand[j + 1] = v;
-    }
-    double fx = 0.0, fy = 0.0, fz = 0.0;
-    for (int i = 0; i < nc; ++i) {
-        const int q = cand[i];
-        const double dx = dsub(x, PCOL(st, np, 0, q));
-        const double dy = dsub(y, PCOL(st, np, 1, q));
-        const double dz = dsub(z, PCOL(st, np, 2, q));
-        const double dist = __dsqrt_rn(sq3(dx, dy, dz));
-        const double hgap = dsub(dist, dmul(2.0, radius));
-        const double overlap = (hgap < 0.0) ? -hgap : 0.0;
-        const double factor = __ddiv_rn(dsub(min_gap, hgap), min_gap);
-        const double lub = dmul(coeff, dadd(__ddiv_rn(dmul(factor, factor), ph.stf0),
-                                            __ddiv_rn(overlap, dmul(min_gap, ph.stf1))));
-        fx = dadd(fx, dmul(lub, __ddiv_rn(dx, dist)));
-        fy = dadd(fy, dmul(lub, __ddiv_rn(dy, dist)));
-        fz = dadd(fz, dmul(lub, __ddiv_rn(dz, dist)));
-        if (q > p) {
-            const int slot = atomicAdd(&status->ncontacts, 1);
-            if (slot < pb.pair_cap) { pb.pair_p[slot] = p; pb.pair_q[slot] = q; }
+    if (nc > MAX_CAND) nc = MAX_CAND;
+    if (lane == 0) {
+        if (ncand > MAX_CAND) atomicOr(&status->contact_overflow, 1);
+        for (int i = 1; i < nc; ++i) {
+            const int v = cand[i];
+            int j = i - 1;
+            while (j >= 0 && cand[j] > v) { cand[j + 1] = cand[j]; --j; }
+            cand[j + 1] = v;
         }
     }
-    // walls (pforces.cu:40-76)
-    double wfx = 0.0, wfy = 0.0, wfz = 0.0;
-    const double gaps[6] = {dsub(x, radius), dsub(dsub((double)geo.lx, x), radius),
-                            dsub(y, radius), dsub(dsub((double)geo.ly, y), radius),
-                            dsub(z, radius), dsub(dsub((double)geo.lz, z), radius)};
+    __syncwarp();
+    double fx = 0.0, fy = 0.0, fz = 0.0;
+    for (int i0 = 0; i0 < nc; i0 += 32) {
+        const int i = i0 + lane, q = cand[i < nc ? i : 0];
+        double px = 0.0, py = 0.0, pz = 0.0;
+        if (i < nc) {
+            const double dx = dsub(x, PCOL(st, np, 0, q));
+            const double dy = dsub(y, PCOL(st, np, 1, q));
+            const double dz = dsub(z, PCOL(st, np, 2, q));
+            const double dist = __dsqrt_rn(sq3(dx, dy, dz));
+            const double hgap = dsub(dist, dmul(2.0, radius));
+            const double overlap = (hgap < 0.0) ? -hgap : 0.0;
+            const double factor = __ddiv_rn(dsub(min_gap, hgap), min_gap);
+            const double lub = dmul(coeff, dadd(__ddiv_rn(dmul(factor, factor), ph.stf0),
+                                                __ddiv_rn(overlap, dmul(min_gap, ph.stf1))));
+            px = dmul(lub, __ddiv_rn(dx, dist));
+            py = dmul(lub, __ddiv_rn(dy, dist));
+            pz = dmul(lub, __ddiv_rn(dz, dist));
+        }
+        for (int k = 0; k < min(32, nc - i0); ++k) {
+            fx = dadd(fx, __shfl_sync(0xffffffffu, px, k));
+            fy = dadd(fy, __shfl_sync(0xffffffffu, py, k));
+            fz = dadd(fz, __shfl_sync(0xffffffffu, pz, k));
+        }
+        const unsigned first = __ballot_sync(0xffffffffu, i < nc && q > p);
+        int base = 0;
+        if (lane == 0 && first) base = atomicAdd(&status->ncontacts, __popc(first));
+        const int slot = __shfl_sync(0xffffffffu, base, 0) + __popc(first & ((1u << lane) - 1u));
+        if ((first >> lane & 1u) && slot < pb.pair_cap) { pb.pair_p[slot] = p; pb.pair_q[slot] = q; }
+    }
+    // walls (pforces.cu:40-76), lane k < 6: normals +x, -x, +y, -y, +z, -z
+    const int axis = lane >> 1;
+    const double at = axis == 0 ? x : (axis == 1 ? y : z);
+    const int extent = axis == 0 ? geo.lx : (axis == 1 ? geo.ly : geo.lz);
+    const double gap = dsub(lane & 1 ? dsub((double)extent, at) : at, radius);
     const double mgw = ph.min_gap_w;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        const double gap = gaps[k];
-        if (gap >= mgw) continue;
+    const bool touches = lane < 6 && !(gap >= mgw);
+    double push = 0.0;
+    if (touches) {
         const double overlap = (gap < 0.0) ? -gap : 0.0;
         const double factor = __ddiv_rn(dsub(mgw, gap), mgw);
         const double lub = dmul(coeff, dadd(__ddiv_rn(dmul(factor, factor), ph.stf0_w),
                                             __ddiv_rn(overlap, dmul(mgw, ph.stf1_w))));
-        // wall normals +x, -x, +y, -y, +z, -z; the zero components add +0.0 and are skipped
-        const double sgn = (k & 1) ? -1.0 : 1.0;
-        if (k < 2) wfx = dadd(wfx, dmul(lub, sgn));
-        else if (k < 4) wfy = dadd(wfy, dmul(lub, sgn));
-        else wfz = dadd(wfz, dmul(lub, sgn));
+        push = lane & 1 ? -lub : lub;
     }
-    pb.cF[p] = dadd(fx, wfx);
-    pb.cF[np + p] = dadd(fy, wfy);
-    pb.cF[2 * np + p] = dadd(fz, wfz);
+    // lane a < 3 adds axis a's two walls, then the pairs' force to them; what does not touch adds nothing
+    const unsigned walls = __ballot_sync(0xffffffffu, touches);
+    const int a = lane < 3 ? lane : 0;
+    const double lo = __shfl_sync(0xffffffffu, push, 2 * a), hi = __shfl_sync(0xffffffffu, push, 2 * a + 1);
+    double wf = 0.0;
+    if (walls >> (2 * a) & 1u) wf = dadd(wf, lo);
+    if (walls >> (2 * a + 1) & 1u) wf = dadd(wf, hi);
+    if (lane < 3) pb.cF[lane * np + p] = dadd(lane == 0 ? fx : (lane == 1 ? fy : fz), wf);
 }
 
 __global__ void __launch_bounds__(32 * CONTACT_WARPS) k_contact_force(const Geo geo, const Phys ph,
@@ -1183,8 +1197,10 @@ __global__ void __launch_bounds__(NT) k_new_fluid(const Geo geo, const Phys ph, 
 // wall-processed population in slot (opp(ip), n) (bounce-back: f*_ip itself; the Dirichlet image of
 // g*_ip at a pure x exit is inverted with the step's density at n, which the step kernel wrote to
 // rho).  The kernel is a chain of loads and of FP64 additions (64 cycles each for the warp): the
-// owners of all neighbours are looked at at once, a lane each, the populations are loaded four
-// neighbours at a time, and the node macros are only formed on steps that output them.
+// owners of all neighbours are looked at at once, a lane each, the populations of eight neighbours (and
+// the eight beyond them) are loaded before the first is converted, which would wait for it (with the
+// contact forces' lanes: 128x128x64 with 40 spheres 168 -> 159 us per step in FP32, 64x64x32 with 9
+// 82 -> 79), and the node macros are only formed on steps that output them.
 template <int MODE>
 __device__ __forceinline__ void refill_compute_body(const Geo &geo, const Phys &ph, const PartBuffers &pb,
                                                     const int *owner_prev, const void *f_, const void *g_,
@@ -1226,42 +1242,49 @@ __device__ __forceinline__ void refill_compute_body(const Geo &geo, const Phys &
             const int ip = lane;
             const double w = dweight_rt(ip);
             const int cxp = dcx_rt(ip), cyp = dcy_rt(ip), czp = dcz_rt(ip), op = dopp_rt(ip);
-            auto load = [&](long long slot, int xs) {
-                return widen(is_g ? ST::ld_g(pops + slot, w, gshift(ph, xs)) : ST::ld_f(pops + slot, w, ph.t0));
+            // where the step left f*_ip or g*_ip of the previous-step fluid node n = node + m c_k
+            struct At {
+                long long n, slot;
+                int xs;
+                bool image;
             };
-            // f*_ip or g*_ip of the previous-step fluid node n = (xn, yn, zn)
-            auto collided = [&](long long n, int xn, int yn, int zn) -> double {
-                if (!odd) return load((long long)op * L + n, xn);
-                const int xd = xn + cxp, yd = yn + cyp, zd = zn + czp;
-                if (xd >= 0 && xd < geo.lx && yd >= 0 && yd < geo.ly && zd >= 0 && zd < geo.lz)
-                    return load((long long)ip * L + (long long)zd * geo.lxy + (long long)yd * geo.lx + xd, xd);
-                double v = load((long long)op * L + n, xn);
+            auto at = [&](int k, int m) {
+                const int c1 = m * dcx_rt(k), c2 = m * dcy_rt(k), c3 = m * dcz_rt(k);
+                const int xn = ix + c1, xd = xn + cxp, yd = iy + c2 + cyp, zd = iz + c3 + czp;
                 const bool ox = xd < 0 || xd >= geo.lx, oyz = yd < 0 || yd >= geo.ly || zd < 0 || zd >= geo.lz;
-                if (is_g && ox && !oyz) v = wall_image(v, w, xd < 0 ? ph.thot : ph.tcold, rho[n]);
+                const bool on = odd && !ox && !oyz;
+                At r;
+                r.n = idx + (long long)c3 * geo.lxy + (long long)c2 * geo.lx + c1;
+                r.slot = on ? (long long)ip * L + r.n + (long long)czp * geo.lxy + (long long)cyp * geo.lx + cxp
+                            : (long long)op * L + r.n;
+                r.xs = on ? xd : xn;
+                r.image = is_g && odd && ox && !oyz;
+                return r;
+            };
+            auto value_of = [&](const At &r, const S &raw) -> double {
+                double v = widen(is_g ? ST::ld_g(&raw, w, gshift(ph, r.xs)) : ST::ld_f(&raw, w, ph.t0));
+                if (r.image) v = wall_image(v, w, cxp < 0 ? ph.thot : ph.tcold, rho[r.n]);
                 return v;
             };
             const int sc = __popc(near_fluid);
             for (unsigned m = near_fluid; m;) {   // ascending neighbours
-                double v1[4], v2[4];
+                constexpr int TOGETHER = 8;
+                S s1[TOGETHER], s2[TOGETHER];
                 unsigned mm = m;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    if (!mm) break;
-                    const int ip2 = __ffs((int)mm) - 1;
-                    mm &= mm - 1;
-                    const int cx2 = dcx_rt(ip2), cy2 = dcy_rt(ip2), cz2 = dcz_rt(ip2);
-                    const long long off = (long long)cz2 * geo.lxy + (long long)cy2 * geo.lx + cx2;
-                    v1[k] = collided(idx + off, ix + cx2, iy + cy2, iz + cz2);
-                    if (next_fluid >> ip2 & 1u)
-                        v2[k] = collided(idx + 2 * off, ix + 2 * cx2, iy + 2 * cy2, iz + 2 * cz2);
+                for (int k = 0; k < TOGETHER; ++k, mm &= mm - 1) {
+                    const int ip2 = mm ? __ffs((int)mm) - 1 : 0;   // none left: the node's own, not used
+                    s1[k] = pops[at(ip2, 1).slot];
+                    s2[k] = pops[at(ip2, next_fluid >> ip2 & 1u ? 2 : 1).slot];
                 }
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
+                for (int k = 0; k < TOGETHER; ++k) {
                     if (!m) break;
                     const int ip2 = __ffs((int)m) - 1;
                     m &= m - 1;
-                    if (next_fluid >> ip2 & 1u) value += 2.0 * v1[k] - v2[k];
-                    else value += v1[k];
+                    const double v1 = value_of(at(ip2, 1), s1[k]);
+                    if (next_fluid >> ip2 & 1u) value += 2.0 * v1 - value_of(at(ip2, 2), s2[k]);
+                    else value += v1;
                 }
             }
             if (sc == 0) {
