@@ -37,8 +37,9 @@ __device__ __forceinline__ void pdl_trigger()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 #endif
 }
+// allowed: false for an ordinary launch
 template <typename... KArgs, typename... Args>
-cudaError_t pdl_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args)
+cudaError_t pdl_launch_if(bool allowed, void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -47,10 +48,16 @@ cudaError_t pdl_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStre
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = RBTP_USE_PDL;
+    attr[0].val.programmaticStreamSerializationAllowed = RBTP_USE_PDL && allowed;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t pdl_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args)
+{
+    return pdl_launch_if(true, kernel, grid, block, st, args...);
 }
 
 // ------------------------------------------------------------------------------------------------
