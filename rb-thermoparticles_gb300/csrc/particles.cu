@@ -1683,8 +1683,10 @@ __global__ void __launch_bounds__(NT) k_mark_b(const CavDesc *desc, const int2 *
 template <bool F32Q, int NT>
 // 128-thread CTAs are held to 48 registers (10 resident per SM): the descriptor fields the batched
 // body reads cost registers the single-cavity kernel takes from its parameters, and at 72 registers
-// only 7 CTAs fit (the 256-cavity ensemble step is 1 % faster with the small spill this leaves)
-__global__ void __launch_bounds__(NT, NT == LINK_NARROW ? 10 : 1) k_link_fill_b(const CavDesc *desc, const int2 *pmap)
+// only 7 CTAs fit (the 256-cavity ensemble step is 1 % faster with the small spill this leaves);
+// 512-thread CTAs to 64, for two per SM: with 96 one fits, and the 219 spheres of a batch of 32 members
+// took a second wave (0.448 -> 0.434 ms per step in FP32, 1.518 -> 1.507 in FP64)
+__global__ void __launch_bounds__(NT, NT == LINK_NARROW ? 10 : 2) k_link_fill_b(const CavDesc *desc, const int2 *pmap)
 {
     pdl_wait();
     pdl_trigger();
