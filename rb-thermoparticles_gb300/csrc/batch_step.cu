@@ -187,8 +187,8 @@ __global__ void __launch_bounds__(2 * STEP64_NODES, STEP64_BLOCKS)
         const int z1 = min(tl.w + BATCH_TILE_Z, sgeo.lz);
         const bool odd = d.phase == PHASE_SWAPPED;
         for (int iz = tl.w; iz < z1; ++iz) {
-            if (odd) step_node64<true, false>(sgeo, sk, b, d.out, ix, iy, iz, active, smem);
-            else step_node64<false, false>(sgeo, sk, b, d.out, ix, iy, iz, active, smem);
+            if (odd) step_node64<true, false, 1>(sgeo, sk, b, d.out, ix, iy, iz, active, smem);
+            else step_node64<false, false, 1>(sgeo, sk, b, d.out, ix, iy, iz, active, smem);
         }
     }
 }

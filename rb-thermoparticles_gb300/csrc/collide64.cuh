@@ -188,9 +188,9 @@ __host__ __device__ __forceinline__ void coef64_g(double (&c)[NCOEF64], const Sr
 }
 
 // The collided population om val + w X of every place 9 s + q, handed to out(s, r[9]) slab by slab
-// (s = cy + 1).  `weighted` is that of tops64.  False, with nothing handed out, where a coefficient
-// is too large for the grids (or not finite).
-template <class Out>
+// (s = cy + 1; UNROLL slabs per round of the loop).  `weighted` is that of tops64.  False, with nothing
+// handed out, where a coefficient is too large for the grids (or not finite).
+template <int UNROLL, class Out>
 __host__ __device__ __forceinline__ bool relax64(const double *val, int stride, double omega, uint32_t weighted,
                                                  const double (&c)[NCOEF64], Out &&out)
 {
@@ -205,7 +205,7 @@ __host__ __device__ __forceinline__ bool relax64(const double *val, int stride, 
 #pragma unroll
     for (int k = 0; k < NCOEF64; ++k) a[k] = fx_from(c[k], grid);
     const FxFactor om = fx_factor(omega);
-#pragma unroll 1
+#pragma unroll UNROLL
     for (int s = 0; s < 3; ++s, val += 9 * stride) {
         // the polynomial of this slab: cy = s - 1
         int64_t k0 = a[1], kx = a[8], kz = a[10], kxx = a[2], kxz = a[6];

@@ -41,9 +41,9 @@ __global__ void __launch_bounds__(128, RBTP_STEP_MINB)
 }
 
 // Blocks of 32 consecutive nodes of a plane, f and g (step_node64.cuh).
-template <bool ODD, int OUT>
+template <bool ODD, bool COL, int UNROLL>
 __global__ void __launch_bounds__(2 * STEP64_NODES, STEP64_BLOCKS)
-    k_step64(const Geo geo, const Phys ph, const StepBuffers b)
+    k_step64(const Geo geo, const Phys ph, const StepBuffers b, const int out)
 {
     __shared__ double smem[STEP64_DOUBLES];
     pdl_wait();
@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(2 * STEP64_NODES, STEP64_BLOCKS)
     const unsigned n = blockIdx.x * STEP64_NODES + threadIdx.x, lxy = (unsigned)geo.lxy;
     int ix, iy;
     plane_node(geo, min(n, lxy - 1u), ix, iy);
-    step_node64<ODD, OUT == OUT_MACROS_COL>(geo, ph.kd, b, OUT, ix, iy, blockIdx.y, n < lxy, smem);
+    step_node64<ODD, COL, UNROLL>(geo, ph.kd, b, out, ix, iy, blockIdx.y, n < lxy, smem);
 }
 
 // Stream-only export: the post-streaming populations f(n) of the reference (its d_f / d_g after a
@@ -282,18 +282,22 @@ cudaError_t launch_step_mode(bool odd, int out, const Geo &geo, const Phys &ph,
     // touch no neighbour, run best in 64-node rows (0.583 against 0.596 ms for 32-wide rows).
     if constexpr (MODE == RBTP_STORE_F64) {
         const dim3 grd((unsigned)((geo.lxy + STEP64_NODES - 1) / STEP64_NODES), geo.lz);
-#define RBTP_STEP_CASE(P, O)                                                                                     \
-    if (odd == P && out == O)                                                                                    \
-        return pdl_launch(k_step64<P, O>, grd, dim3(STEP64_NODES, 1, 2), st, geo, ph, b);
-        RBTP_STEP_CASE(true, OUT_NONE)
-        RBTP_STEP_CASE(true, OUT_RHO)
-        RBTP_STEP_CASE(true, OUT_MACROS)
-        RBTP_STEP_CASE(true, OUT_MACROS_COL)
-        RBTP_STEP_CASE(false, OUT_NONE)
-        RBTP_STEP_CASE(false, OUT_RHO)
-        RBTP_STEP_CASE(false, OUT_MACROS)
-        RBTP_STEP_CASE(false, OUT_MACROS_COL)
-#undef RBTP_STEP_CASE
+        const dim3 blk(STEP64_NODES, 1, 2);
+        if (out < OUT_NONE || out > OUT_MACROS_COL) return cudaErrorInvalidValue;
+        if (out == OUT_MACROS_COL)
+            return odd ? pdl_launch(k_step64<true, true, 1>, grd, blk, st, geo, ph, b, out)
+                       : pdl_launch(k_step64<false, true, 1>, grd, blk, st, geo, ph, b, out);
+        // A grid of few waves of resident blocks runs at the latency of a block's chain of instructions,
+        // which unrolled slabs shorten; a longer one is bound by throughput, and then the 42 KB of
+        // the odd step (32 KB of the even one) with the loop stay in the instruction caches and its
+        // 58 KB (46 KB) without do not.  Both unrolled | both looped: 32x32x16 10.4 | 11.5 us, 48x48x24
+        // 20.3 | 21.9, 64x64x32 43.3 | 44.5 (only the odd step unrolled: 42.9), 80x80x40 85.6 | 81.3,
+        // 128x128x64 310 | 284, 320x320x160 4.57 | 4.21 ms.
+        constexpr long long WAVE = 152LL * STEP64_BLOCKS * STEP64_NODES;
+        if (odd && geo.L <= 3 * WAVE) return pdl_launch(k_step64<true, false, 3>, grd, blk, st, geo, ph, b, out);
+        if (!odd && geo.L <= 2 * WAVE) return pdl_launch(k_step64<false, false, 3>, grd, blk, st, geo, ph, b, out);
+        return odd ? pdl_launch(k_step64<true, false, 1>, grd, blk, st, geo, ph, b, out)
+                   : pdl_launch(k_step64<false, false, 1>, grd, blk, st, geo, ph, b, out);
     } else {
         dim3 blk(32, 4, 1);
         if (MODE == RBTP_STORE_F16S)

@@ -93,14 +93,15 @@ __device__ __forceinline__ double *slot_at(double *base, unsigned i8, unsigned L
 // passing through registers, and are read from there where they are used, and f and g of a node
 // belong to two threads, which exchange the moments: six warps per scheduler.  The code loops over the
 // three slabs of directions: unrolled, its 75 KB did not stay in the instruction caches.  Measured
-// at 320x320x160: 4.4 ms per step, 13.1 ms with every sum on the FP64 pipe (424 FP64 instructions
+// at 320x320x160: 4.2 ms per step, 13.1 ms with every sum on the FP64 pipe (424 FP64 instructions
 // per node there, 77 here; 880 B per node at the copy bandwidth would take 2.2 ms); at 64x64x32 43
 // against 118 us.  What bounds it now is the latency of the chain load - integer sums - FP64
 // coefficients - integer sums with the warps that fit (integer pipe 61 %, FP64 pipe 48 % busy).  `out`
-// selects the outputs (StepOut; COL: also the post-collision copies), `smem` is the block's shared
-// memory.  Threads that are not `active` only take part in the barriers; they read the slots of the
-// node they are given (which must exist).
-template <bool ODD, bool COL>
+// selects the outputs (StepOut; COL: also the post-collision copies; a kernel for each value had the
+// compiler unroll some, see the choice of UNROLL, the slabs per round of the collision's loop, in
+// lbm_step.cu), `smem` is the block's shared memory.  Threads that are not `active` only take part in
+// the barriers; they read the slots of the node they are given (which must exist).
+template <bool ODD, bool COL, int UNROLL>
 __device__ __forceinline__ void step_node64(const Geo &geo, const StepK<double> &K, const StepBuffers &b, int out,
                                             int ix, int iy, int iz, bool active, double *smem)
 {
@@ -255,7 +256,7 @@ __device__ __forceinline__ void step_node64(const Geo &geo, const StepK<double> 
         if (ODD && is_g && out_x != 0u) pop[p * T] = r;
     };
     const double omega = is_g ? K.omc : K.om;
-    if (!relax64(pop, T, omega, tops.weighted, c, [&](int s, const double(&r)[9]) {
+    if (!relax64<UNROLL>(pop, T, omega, tops.weighted, c, [&](int s, const double(&r)[9]) {
             if (active) {
 #pragma unroll
                 for (int q = 0; q < 9; ++q) scatter(s, q, r[q]);

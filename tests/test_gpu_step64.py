@@ -112,3 +112,22 @@ def test_batched_fp64_members_of_ragged_sizes_match_single_runs(lib_built):
             b.close()
     for x, y in zip(*runs):
         assert np.array_equal(x[0], y[0]) and np.array_equal(x[1], y[1])
+
+
+# 57 x 64 x 32 and 57 x 64 x 48 nodes: the last grids that take the unrolled even and odd step
+@pytest.mark.parametrize("lz", [32, 33, 48, 49])
+def test_both_unrollings_give_the_same_bits(lib_built, lz):
+    fg = _populations(57, 64, lz, lz, 5)
+    runs = []
+    for batched in (False, True):
+        s = Solver(W.config("plain_fp64", lx=57, ly=64, lz=lz))
+        s.load_state(*fg, None)
+        if batched:
+            b = Batch(0)
+            b.add(s)
+            b.step(3)
+            b.close()
+        else:
+            s.step(3)
+        runs.append(s.fg())
+    assert np.array_equal(runs[0][0], runs[1][0]) and np.array_equal(runs[0][1], runs[1][1])
