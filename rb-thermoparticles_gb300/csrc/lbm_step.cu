@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(128, RBTP_STEP_MINB)
 }
 
 // Blocks of 32 consecutive nodes of a plane, f and g (step_node64.cuh).
-template <bool ODD, bool COL, int UNROLL>
+template <bool ODD, int OUT, int UNROLL>
 __global__ void __launch_bounds__(2 * STEP64_NODES, STEP64_BLOCKS)
     k_step64(const Geo geo, const Phys ph, const StepBuffers b, const int out)
 {
@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(2 * STEP64_NODES, STEP64_BLOCKS)
     const unsigned n = blockIdx.x * STEP64_NODES + threadIdx.x, lxy = (unsigned)geo.lxy;
     int ix, iy;
     plane_node(geo, min(n, lxy - 1u), ix, iy);
-    step_node64<ODD, COL, UNROLL>(geo, ph.kd, b, out, ix, iy, blockIdx.y, n < lxy, smem);
+    step_node64<ODD, OUT == OUT_MACROS_COL, UNROLL>(geo, ph.kd, b, OUT == OUT_RUNTIME ? out : OUT, ix, iy, blockIdx.y, n < lxy, smem);
 }
 
 // Stream-only export: the post-streaming populations f(n) of the reference (its d_f / d_g after a
@@ -285,19 +285,24 @@ cudaError_t launch_step_mode(bool odd, int out, const Geo &geo, const Phys &ph,
         const dim3 blk(STEP64_NODES, 1, 2);
         if (out < OUT_NONE || out > OUT_MACROS_COL) return cudaErrorInvalidValue;
         if (out == OUT_MACROS_COL)
-            return odd ? pdl_launch(k_step64<true, true, 1>, grd, blk, st, geo, ph, b, out)
-                       : pdl_launch(k_step64<false, true, 1>, grd, blk, st, geo, ph, b, out);
-        // A grid of few waves of resident blocks runs at the latency of a block's chain of instructions,
-        // which unrolled slabs shorten; a longer one is bound by throughput, and then the 42 KB of
-        // the odd step (32 KB of the even one) with the loop stay in the instruction caches and its
-        // 58 KB (46 KB) without do not.  Both unrolled | both looped: 32x32x16 10.4 | 11.5 us, 48x48x24
-        // 20.3 | 21.9, 64x64x32 43.3 | 44.5 (only the odd step unrolled: 42.9), 80x80x40 85.6 | 81.3,
-        // 128x128x64 310 | 284, 320x320x160 4.57 | 4.21 ms.
+            return odd ? pdl_launch(k_step64<true, OUT_MACROS_COL, 1>, grd, blk, st, geo, ph, b, out)
+                       : pdl_launch(k_step64<false, OUT_MACROS_COL, 1>, grd, blk, st, geo, ph, b, out);
+        // A grid of up to three waves of resident blocks runs at the latency of a block's chain of
+        // instructions, which unrolled slabs and fixed outputs shorten; a longer one is bound by
+        // throughput, and then the 42 KB of the odd step (32 KB of the even one) with the loop stay in
+        // the instruction caches and its 58 KB (45 KB) without do not.  Short chain | loop: 32x32x16
+        // 10.2 | 11.5 us, 48x48x24 20.0 | 21.9, 64x64x32 42.3 | 44.5, but 80x80x40 85.6 | 81.3, 128x128x64
+        // 310 | 284, 320x320x160 4.57 | 4.21 ms.
         constexpr long long WAVE = 152LL * STEP64_BLOCKS * STEP64_NODES;
-        if (odd && geo.L <= 3 * WAVE) return pdl_launch(k_step64<true, false, 3>, grd, blk, st, geo, ph, b, out);
-        if (!odd && geo.L <= 2 * WAVE) return pdl_launch(k_step64<false, false, 3>, grd, blk, st, geo, ph, b, out);
-        return odd ? pdl_launch(k_step64<true, false, 1>, grd, blk, st, geo, ph, b, out)
-                   : pdl_launch(k_step64<false, false, 1>, grd, blk, st, geo, ph, b, out);
+        if (geo.L <= 3 * WAVE) {
+            if (out == OUT_NONE)
+                return odd ? pdl_launch(k_step64<true, OUT_NONE, 3>, grd, blk, st, geo, ph, b, out)
+                           : pdl_launch(k_step64<false, OUT_NONE, 3>, grd, blk, st, geo, ph, b, out);
+            return odd ? pdl_launch(k_step64<true, OUT_RUNTIME, 3>, grd, blk, st, geo, ph, b, out)
+                       : pdl_launch(k_step64<false, OUT_RUNTIME, 3>, grd, blk, st, geo, ph, b, out);
+        }
+        return odd ? pdl_launch(k_step64<true, OUT_RUNTIME, 1>, grd, blk, st, geo, ph, b, out)
+                   : pdl_launch(k_step64<false, OUT_RUNTIME, 1>, grd, blk, st, geo, ph, b, out);
     } else {
         dim3 blk(32, 4, 1);
         if (MODE == RBTP_STORE_F16S)

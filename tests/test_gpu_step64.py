@@ -114,8 +114,7 @@ def test_batched_fp64_members_of_ragged_sizes_match_single_runs(lib_built):
         assert np.array_equal(x[0], y[0]) and np.array_equal(x[1], y[1])
 
 
-# 57 x 64 x 32 and 57 x 64 x 48 nodes: the last grids that take the unrolled even and odd step
-@pytest.mark.parametrize("lz", [32, 33, 48, 49])
+@pytest.mark.parametrize("lz", [48, 49])   # 57 x 64 x 48 nodes: the last grid that takes the unrolled step
 def test_both_unrollings_give_the_same_bits(lib_built, lz):
     fg = _populations(57, 64, lz, lz, 5)
     runs = []
