@@ -41,26 +41,24 @@ FALLBACK_HBM_GBS = 6800.0
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one k_step launch, the mean of one
 # even-step and one odd-step launch of the in-place storage, from one-pass ncu captures of
 # `python bench.py --only production:<storage> --steps 4 --warmup 3` (FP32, shifted FP16: the
-# 320x320x160 workload itself) and `... --only production:f64 --grid 192x192x96 ...` (FP64, 3.1 GB
+# 320x320x160 workload itself) and `... --only production:f64 --grid 128x128x64 ...` (FP64, 0.97 GB
 # per launch, scaled to 16,384,000 nodes by the node count; its reads are exactly 440 B per node,
-# its writes 423 B per node because L2 still holds part of them when the kernel ends).  The
-# captures' summary is kept with the other ncu summaries.  Algorithmic bytes per launch:
+# its writes 466 (even) and 497 B (odd)).  The captures' summary is kept with the other ncu summaries.  Algorithmic bytes per launch:
 # 16,384,000 nodes x bytes_per_node.
 NCU_DRAM_BYTES = {
     "f32": ((3.607174144e9 + 3.569068288e9) + (3.604580352e9 + 3.557273600e9)) / 2,
     "f16s": ((1.835989248e9 + 1.781190144e9) + (1.835062016e9 + 1.772242432e9)) / 2,
-    "f64": ((1.558169344e9 + 1.497404672e9) + (1.557334528e9 + 1.492732416e9)) / 2 * 16384000 / (192 * 192 * 96),
+    "f64": ((0.461615360e9 + 0.521240832e9) + (0.461455360e9 + 0.489164800e9)) / 2 * 16384000 / (128 * 128 * 64),
 }
 
 
-# FP64 work of one FP64 k_step node update, from one ncu capture of an odd and an even launch
-# (k_step<0,1,0>, k_step<0,0,0>) on 128x128x64 (1,048,576 nodes) with `python bench.py --only
-# production:f64 --grid 128x128x64 --steps 4 --warmup 3`:
+# FP64 work of one FP64 node update (most of whose sums run on the integer units), from one ncu
+# capture of an odd and an even launch of k_step64 on 128x128x64 (1,048,576 nodes) with `python bench.py
+# --only production:f64 --grid 128x128x64 --steps 4 --warmup 3`:
 # smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}_pred_on.sum per node, odd / even:
-# 167.41 / 167.00 DFMA, 189.15 / 189.00 DADD, 68.23 / 68.00 DMUL, i.e. 424.4 FP64 arithmetic
-# instructions (426.4 with the FP64 compares and conversions) and 591.6 flops (an FMA counts 2)
-# per node on average.
-_FP64_DFMA, _FP64_DADD, _FP64_DMUL = (167.41 + 167.00) / 2, (189.15 + 189.00) / 2, (68.23 + 68.00) / 2
+# 25.28 / 25.00 DFMA, 5.28 / 5.00 DADD, 44.28 / 44.00 DMUL, i.e. 74.4 FP64 instructions and 99.6 flops
+# (an FMA counts 2) per node on average.
+_FP64_DFMA, _FP64_DADD, _FP64_DMUL = (25.28 + 25.00) / 2, (5.28 + 5.00) / 2, (44.28 + 44.00) / 2
 FP64_FLOPS_PER_NODE = 2 * _FP64_DFMA + _FP64_DADD + _FP64_DMUL
 FP64_INST_PER_NODE = _FP64_DFMA + _FP64_DADD + _FP64_DMUL
 
@@ -177,7 +175,7 @@ def time_variant(torch, name, storage, steps, warmup, dist=None, keep_state=Fals
     out = {"workload": name + "".join(f" {k}={v}" for k, v in over.items()),
            "storage": ["f64", "f32", "f16s"][storage], "ms_per_step": ms / steps,
            "mlups": L * steps / (ms * 1e-3) / 1e6, "nodes": L,
-           "launches_per_step": 1 if not cfg.activate_particles else 14}
+           "launches_per_step": 1 if not cfg.activate_particles else 13}
     if cfg.activate_particles:
         out["npart"] = s.npart
     if keep_state:
@@ -593,7 +591,7 @@ def run_ours(args) -> dict:
     for v in (head, fp64, f16, p64, p32):
         if "error" not in v:
             v["roofline"] = roof(v)
-    # the FP64 path is bound by the FP64 pipe: its compute roofline against the measured FMA rate
+    # the FP64 path's share of the measured FMA rate (its sums run on the integer units)
     from rbtp import fp64_fma_rate
     dfma = guarded(fp64_fma_rate)
     fp64_compute = None

@@ -4,9 +4,10 @@
 // device so that the whole step can be captured once in a CUDA graph and replayed.
 //
 // Tile table: int4 (cavity, tile_x, tile_y, z) for every TX x TY tile of every cavity (TY = 1: runs of
-// TX consecutive nodes of the plane, tile_x-th), packed cavity after cavity.  The persistent grid (chosen by the host autotuner, a multiple of the SM
-// count) walks the table with a grid stride, so small and large cavities share the machine without
-// per-cavity launches.
+// TX consecutive nodes of the plane, tile_x-th), packed cavity after cavity.  The persistent grid
+// (chosen by the host autotuner, a multiple of the SM count) walks the table with a grid stride, so
+// small and large cavities share the machine without per-cavity launches.  FP64 walks it in parts of
+// 32 nodes of a tile.
 #include <algorithm>
 
 #include "step_node.cuh"
@@ -64,7 +65,7 @@ __global__ void k_batch_advance(CavDesc *desc, int n)
 // member's AAOff staged in shared memory, and the face tests from per-node masks (FACE_MASK); see
 // step_node.cuh for what each is worth.  Shifted FP16, bound by instruction issue, takes the output
 // mode at run time, which leaves room in the instruction caches for the odd step's interior path: 32
-// members of 32 to 80 nodes across, per step 0.258 -> 0.250 ms without spheres, 0.402 -> 0.383 ms with
+// members of 32 to 96 nodes across, per step 0.258 -> 0.250 ms without spheres, 0.402 -> 0.383 ms with
 // them.  FP32, bound by memory latency, ran 0.331 -> 0.341 ms with the same (0.338 without the
 // interior path).
 template <int MODE, bool ODD>

@@ -1,6 +1,6 @@
 // lbm_step.cu — fused D3Q27 f+g stream/collide kernel (in-place AA storage) for sm_103a.
 //
-// One thread per lattice node.  The kernel replaces the reference's per-step sequence
+// One thread per lattice node (FP64: two, step_node64.cuh).  The kernel replaces the reference's per-step sequence
 //   macrovar (macrovar.cu:3-34) -> forcing (macrovar.cu:36-47) -> collision_BGK (collision.cu:3-33)
 //   -> f_collide copy -> streaming (streaming.cu:3-23) -> collision_BGK_scalar (collision.cu:35-89)
 //   -> g_collide copy -> streaming_scalar (streaming.cu:25-63)

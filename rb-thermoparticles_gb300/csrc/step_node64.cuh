@@ -12,7 +12,7 @@ namespace rbtp {
 // memory: the 27 populations of thread t at [place][t] (places of collide64.cuh), and what the two
 // threads of a node exchange.  A block is one warp pair, whose shared memory is free again when its
 // slower warp is done (four pairs: 4.65 against 4.45 ms per step at 320x320x160, and 1.41 against
-// 1.35 ms for a batch of 32 members of 32 to 80 nodes across).
+// 1.35 ms for a batch of 32 members of 32 to 96 nodes across).
 constexpr int STEP64_NODES = 32;
 constexpr int STEP64_SWAP = 16;      // doubles exchanged per node
 constexpr int STEP64_DOUBLES = (27 * 2 + STEP64_SWAP) * STEP64_NODES;
