@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(TX * TY, RBTP_BATCH_MINB_LOW)
 
 // FP64: the tiles in parts of 32 consecutive nodes, one warp pair each.
 template <int TX, int TY>
-__global__ void __launch_bounds__(2 * STEP64_NODES, STEP64_BLOCKS)
+__global__ void __launch_bounds__(2 * STEP64_NODES, STEP64_BLOCKS_BATCHED)
     k_step64_batched(const CavDesc *__restrict__ desc, const int4 *__restrict__ tiles, int ntiles)
 {
     pdl_wait();

@@ -41,8 +41,8 @@ __global__ void __launch_bounds__(128, RBTP_STEP_MINB)
 }
 
 // Blocks of 32 consecutive nodes of a plane, f and g (step_node64.cuh).
-template <bool ODD, int OUT, int UNROLL>
-__global__ void __launch_bounds__(2 * STEP64_NODES, STEP64_BLOCKS)
+template <bool ODD, int OUT, int UNROLL, int BLOCKS = STEP64_BLOCKS>
+__global__ void __launch_bounds__(2 * STEP64_NODES, BLOCKS)
     k_step64(const Geo geo, const Phys ph, const StepBuffers b, const int out)
 {
     __shared__ double smem[STEP64_DOUBLES];
@@ -287,19 +287,30 @@ cudaError_t launch_step_mode(bool odd, int out, const Geo &geo, const Phys &ph,
         if (out == OUT_MACROS_COL)
             return odd ? pdl_launch(k_step64<true, OUT_MACROS_COL, 1>, grd, blk, st, geo, ph, b, out)
                        : pdl_launch(k_step64<false, OUT_MACROS_COL, 1>, grd, blk, st, geo, ph, b, out);
-        // A grid of up to three waves of resident blocks runs at the latency of a block's chain of
+        // A grid of up to four waves of resident blocks runs at the latency of a block's chain of
         // instructions, which unrolled slabs and fixed outputs shorten; a longer one is bound by
         // throughput, and then the 42 KB of the odd step (32 KB of the even one) with the loop stay in
         // the instruction caches and its 58 KB (45 KB) without do not.  Short chain | loop: 32x32x16
-        // 10.2 | 11.5 us, 48x48x24 20.0 | 21.9, 64x64x32 42.3 | 44.5, but 80x80x40 85.6 | 81.3, 128x128x64
-        // 310 | 284, 320x320x160 4.57 | 4.21 ms.
-        constexpr long long WAVE = 152LL * STEP64_BLOCKS * STEP64_NODES;
-        if (geo.L <= 3 * WAVE) {
-            if (out == OUT_NONE)
-                return odd ? pdl_launch(k_step64<true, OUT_NONE, 3>, grd, blk, st, geo, ph, b, out)
-                           : pdl_launch(k_step64<false, OUT_NONE, 3>, grd, blk, st, geo, ph, b, out);
-            return odd ? pdl_launch(k_step64<true, OUT_RUNTIME, 3>, grd, blk, st, geo, ph, b, out)
-                       : pdl_launch(k_step64<false, OUT_RUNTIME, 3>, grd, blk, st, geo, ph, b, out);
+        // 9.7 | 10.3 us, 64x64x32 40.6 | 42.4, 72x72x36 56.8 | 57.5, but 80x80x40 79.3 | 77.6, 96x96x48
+        // 129.8 | 124.5, 320x320x160 4.34 | 3.99 ms.
+        const long long blocks = (long long)grd.x * grd.y;
+        constexpr long long WAVE = 152LL * STEP64_BLOCKS, WAVE_MOST = 152LL * STEP64_BLOCKS_MOST;
+        if (blocks <= 4 * WAVE) {
+            // More resident blocks with fewer registers where that saves a wave that is more than a
+            // quarter full (9 | 12 blocks: 48x48x24 21.4 | 19.9 us, 60x60x30 36.3 | 35.2; but 40x40x20 16.6 |
+            // 20.1, 56x56x28 29.0 | 30.5, 64x64x32 40.6 | 42.3).
+            const bool most = (blocks + WAVE_MOST - 1) / WAVE_MOST < (blocks - WAVE / 4 + WAVE - 1) / WAVE;
+            auto launch = [&](auto O, auto B) {
+                constexpr int OUT = decltype(O)::value, BLOCKS = decltype(B)::value;
+                return odd ? pdl_launch(k_step64<true, OUT, 3, BLOCKS>, grd, blk, st, geo, ph, b, out)
+                           : pdl_launch(k_step64<false, OUT, 3, BLOCKS>, grd, blk, st, geo, ph, b, out);
+            };
+            constexpr std::integral_constant<int, OUT_NONE> NONE{};
+            constexpr std::integral_constant<int, OUT_RUNTIME> ANY{};
+            constexpr std::integral_constant<int, STEP64_BLOCKS> FEW{};
+            constexpr std::integral_constant<int, STEP64_BLOCKS_MOST> MOST{};
+            if (out == OUT_NONE) return most ? launch(NONE, MOST) : launch(NONE, FEW);
+            return most ? launch(ANY, MOST) : launch(ANY, FEW);
         }
         return odd ? pdl_launch(k_step64<true, OUT_RUNTIME, 1>, grd, blk, st, geo, ph, b, out)
                    : pdl_launch(k_step64<false, OUT_RUNTIME, 1>, grd, blk, st, geo, ph, b, out);

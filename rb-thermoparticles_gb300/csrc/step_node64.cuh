@@ -16,7 +16,11 @@ namespace rbtp {
 constexpr int STEP64_NODES = 32;
 constexpr int STEP64_SWAP = 16;      // doubles exchanged per node
 constexpr int STEP64_DOUBLES = (27 * 2 + STEP64_SWAP) * STEP64_NODES;
-constexpr int STEP64_BLOCKS = 12;    // resident per SM, by registers (80 per thread) and shared memory (18 KB)
+// Resident blocks per SM that the kernels ask registers for: 9 (112 per thread), the best of 8 to 12 where a
+// grid has several waves (320x320x160 at 12 | 11 | 10 | 9 | 8: 4.21 | 4.17 | 4.11 | 3.99 | 4.26 ms per step;
+// 113x97x59 196 | 195 | 177 | 173 | 184 us), 12 (80 per thread, all that shared memory allows) for some
+// short grids (lbm_step.cu), and 8 batched (12 | 10 | 9 | 8 | 7 | 6: 1.35 | 1.20 | 1.19 | 1.15 | 1.17 | 1.27 ms).
+constexpr int STEP64_BLOCKS = 9, STEP64_BLOCKS_MOST = 12, STEP64_BLOCKS_BATCHED = 8;
 
 // eight times the direction index of a place, for loops that are not unrolled, and dir_mask by places
 static __constant__ int c_place_dir8[27] = {200, 72, 168, 144, 32, 112, 208, 80, 176, 136, 24, 104, 48, 0, 40, 120, 8, 88, 192, 64, 160, 128, 16, 96, 184, 56, 152};
@@ -91,10 +95,10 @@ __device__ __forceinline__ double *slot_at(double *base, unsigned i8, unsigned L
 // fast as enough warps keep both busy.  With the 54 populations of a node in registers (255) only two
 // warps fit a scheduler; the populations therefore go from global to shared memory by cp.async, without
 // passing through registers, and are read from there where they are used, and f and g of a node
-// belong to two threads, which exchange the moments: six warps per scheduler.  The code loops over the
+// belong to two threads, which exchange the moments: four and a half warps per scheduler.  The code loops over the
 // three slabs of directions: unrolled, its 75 KB did not stay in the instruction caches.  Measured
-// at 320x320x160: 4.2 ms per step, 13.1 ms with every sum on the FP64 pipe (424 FP64 instructions
-// per node there, 77 here; 880 B per node at the copy bandwidth would take 2.2 ms); at 64x64x32 43
+// at 320x320x160: 4.0 ms per step, 13.1 ms with every sum on the FP64 pipe (424 FP64 instructions
+// per node there, 77 here; 880 B per node at the copy bandwidth would take 2.2 ms); at 64x64x32 41
 // against 118 us.  What bounds it now is the latency of the chain load - integer sums - FP64
 // coefficients - integer sums with the warps that fit (integer pipe 61 %, FP64 pipe 48 % busy).  `out`
 // selects the outputs (StepOut; COL: also the post-collision copies; a kernel for each value had the

@@ -114,12 +114,14 @@ def test_batched_fp64_members_of_ragged_sizes_match_single_runs(lib_built):
         assert np.array_equal(x[0], y[0]) and np.array_equal(x[1], y[1])
 
 
-@pytest.mark.parametrize("lz", [48, 49])   # 57 x 64 x 48 nodes: the last grid that takes the unrolled step
-def test_both_unrollings_give_the_same_bits(lib_built, lz):
-    fg = _populations(57, 64, lz, lz, 5)
+# 64 x 57 nodes are 114 blocks of a plane: 12 and 16 planes take each choice of resident blocks, 48 are
+# the last that the unrolled step takes
+@pytest.mark.parametrize("lz", [12, 16, 48, 49])
+def test_all_variants_give_the_same_bits(lib_built, lz):
+    fg = _populations(64, 57, lz, lz, 5)
     runs = []
     for batched in (False, True):
-        s = Solver(W.config("plain_fp64", lx=57, ly=64, lz=lz))
+        s = Solver(W.config("plain_fp64", lx=64, ly=57, lz=lz))
         s.load_state(*fg, None)
         if batched:
             b = Batch(0)
