@@ -41,14 +41,14 @@ FALLBACK_HBM_GBS = 6800.0
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one k_step launch, the mean of one
 # even-step and one odd-step launch of the in-place storage, from one-pass ncu captures of
 # `python bench.py --only production:<storage> --steps 4 --warmup 3` (FP32, shifted FP16: the
-# 320x320x160 workload itself) and `... --only production:f64 --grid 128x128x64 ...` (FP64, 0.97 GB
+# 320x320x160 workload itself) and `... --only production:f64 --grid 128x128x64 ...` (FP64, 0.90 GB
 # per launch, scaled to 16,384,000 nodes by the node count; its reads are exactly 440 B per node,
-# its writes 466 (even) and 497 B (odd)).  The captures' summary is kept with the other ncu summaries.  Algorithmic bytes per launch:
+# its writes 419 B because L2 still holds part of them when the kernel ends).  The captures' summary is kept with the other ncu summaries.  Algorithmic bytes per launch:
 # 16,384,000 nodes x bytes_per_node.
 NCU_DRAM_BYTES = {
     "f32": ((3.607174144e9 + 3.569068288e9) + (3.604580352e9 + 3.557273600e9)) / 2,
     "f16s": ((1.835989248e9 + 1.781190144e9) + (1.835062016e9 + 1.772242432e9)) / 2,
-    "f64": ((0.461615360e9 + 0.521240832e9) + (0.461455360e9 + 0.489164800e9)) / 2 * 16384000 / (128 * 128 * 64),
+    "f64": ((0.461587712e9 + 0.441035008e9) + (0.461507840e9 + 0.438093312e9)) / 2 * 16384000 / (128 * 128 * 64),
 }
 
 
