@@ -1,0 +1,16 @@
+// The host side of fixed64.cuh and collide64.cuh behind C functions, for test_fx_host.py.
+#include "collide64.cuh"
+
+using namespace rbtp;
+
+extern "C" {
+// v^2 / 6 and the three squares of v = 3 u
+void fxh_vel(const double *u, double *out)
+{
+    const Vel64 v = vel64(u[0], u[1], u[2]);
+    out[0] = v.s;
+    out[1] = v.xx;
+    out[2] = v.yy;
+    out[3] = v.zz;
+}
+}
