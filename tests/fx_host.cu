@@ -13,4 +13,12 @@ void fxh_vel(const double *u, double *out)
     out[2] = v.yy;
     out[3] = v.zz;
 }
+unsigned fxh_grid(double largest) { return fx_grid(fx_mag(largest)); }
+long long fxh_from(double d, unsigned grid) { return fx_from(d, grid); }
+double fxh_to(long long v, unsigned grid, int up) { return fx_to(v, grid, up); }
+long long fxh_times(double k, double d, unsigned grid, int up)
+{
+    const FxFactor f = fx_factor(k);
+    return fx_times(f, d, fx_places(f, grid, up));
+}
 }
