@@ -1,0 +1,40 @@
+"""The FP64 step on values that its integer grids do not take."""
+import numpy as np
+import pytest
+
+from rbtp import RbtpError, Solver, workloads as W
+
+pytestmark = pytest.mark.gpu
+LX, LY, LZ = 34, 5, 4
+MIDDLE, WALL = 2 * LX * LY + 2 * LX + 17, LX * LY + 2 * LX   # an inner node and one at the hot wall
+
+
+def _populations(cfg, seed):
+    """f, g near equilibrium of random velocities and temperatures."""
+    rng = np.random.default_rng(seed)
+    L = cfg.nodes
+    u = 0.1 * rng.uniform(-1, 1, (3, L))
+    rho, t = 1e-3 * rng.uniform(-1, 1, L), rng.uniform(0.1, 1, L)
+    cu = W.CX[:, None] * u[0] + W.CY[:, None] * u[1] + W.CZ[:, None] * u[2]
+    e = 3 * cu + 4.5 * cu * cu - 1.5 * (u * u).sum(0)
+    return W.W[:, None] * (rho + e), W.W[:, None] * t * (1 + e)
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf, 1e200])
+@pytest.mark.parametrize("which,direction", [(0, 0), (0, 1), (0, 20), (1, 0), (1, 5)])
+@pytest.mark.parametrize("node", [MIDDLE, WALL])
+def test_a_non_finite_population_reaches_the_populations_that_it_reaches_in_plain_fp64(
+        lib_built, oracle_mod, which, direction, value, node):
+    cfg = W.config("plain_fp64", lx=LX, ly=LY, lz=LZ)
+    fg = _populations(cfg, 1)
+    fg[which][direction, node] = value
+    s, o = Solver(cfg), oracle_mod.Oracle(cfg)
+    for x in (s, o):
+        x.load_state(fg[0].reshape(-1), fg[1].reshape(-1), None)
+    for _ in range(3):
+        with pytest.raises(RbtpError) as e:
+            s.step(1)
+        assert e.value.status == -4
+        o.step(1)
+        for a, b in zip(s.fg(), o.fg()):
+            assert np.array_equal(np.isfinite(a), np.isfinite(b))
