@@ -33,21 +33,6 @@ __host__ __device__ __forceinline__ double fx_twice(double d)
     const uint32_t hi = fx_hi(d);
     return fx_double(hi + ((hi & 0x7fffffffu) < 0x7ff00000u ? 1u << 20 : 0u), fx_lo(d));
 }
-// a / b, b not near the ends of the exponent range: Newton's iteration for 1/b from the hardware's
-// approximation, third order, and one correction of the quotient by its remainder.
-__host__ __device__ __forceinline__ double fx_quotient(double a, double b)
-{
-#ifdef __CUDA_ARCH__
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
-    const double e = fma(-b, r, 1.0);
-    r = fma(r, fma(e, e, e), r);
-    const double q = a * r;
-    return fma(r, fma(-b, q, a), q);
-#else
-    return a / b;
-#endif
-}
 
 // Weights in units of 1/108: exponent of class c (number of nonzero components).
 __host__ __device__ constexpr int up64(int c) { return 5 - 2 * c; }
@@ -171,7 +156,7 @@ __host__ __device__ __forceinline__ Src64 src64(double rho, double ux, double uy
     s.p = pt * (0.5 * W108);
     s.pr = fma(s.p, rho, s.p);
     s.rest = pt * rho;
-    const double rgd = fx_quotient(rho, fma(rho, 1.0 / 3.0, K.gd0)), c2 = rgd * K.Rcw2;
+    const double rgd = rho / fma(rho, 1.0 / 3.0, K.gd0), c2 = rgd * K.Rcw2;
     s.x = fma(c2, fma(-phi, ux, kx), K.Rcw * Fx * phi * (3.0 - rgd));
     s.y = c2 * fma(-phi, uy, ky);
     s.z = c2 * fma(-phi, uz, kz);

@@ -38,3 +38,30 @@ def test_a_non_finite_population_reaches_the_populations_that_it_reaches_in_plai
         o.step(1)
         for a, b in zip(s.fg(), o.fg()):
             assert np.array_equal(np.isfinite(a), np.isfinite(b))
+
+
+def _around(a, r):
+    """The largest |a| over the nodes within r of each node, and over the directions."""
+    m = np.abs(a).max(0).reshape(LZ, LY, LX)
+    for axis in range(3):
+        pad = np.pad(m, [(r, r) if k == axis else (0, 0) for k in range(3)])
+        m = np.max([np.take(pad, range(d, d + m.shape[axis]), axis) for d in range(2 * r + 1)], 0)
+    return m.reshape(-1)
+
+
+@pytest.mark.parametrize("rho", [-0.9, -0.3, -1e-8, 1e-300, 1e-8, 0.7, 40.0, 3e4])
+@pytest.mark.parametrize("prandtl", [0.02, 0.71, 50.0])
+def test_density_over_the_denominator_of_the_scalar_source(lib_built, oracle_mod, rho, prandtl):
+    """rho / (rho / 3 + 2 tauc / 3) of the g source, for densities and diffusivities far from any flow's.  The
+    source's terms are a few times the node's largest g, and its rounding and the sums' are some ten
+    of 2^-53 each: 5e-15 of the largest around."""
+    cfg = W.config("plain_fp64", lx=LX, ly=LY, lz=LZ, prandtl=prandtl, visc=0.02)
+    f, g = _populations(cfg, 5)
+    f += W.W[:, None] * rho * np.random.default_rng(6).uniform(0.5, 1, cfg.nodes)
+    s, o = Solver(cfg), oracle_mod.Oracle(cfg)
+    for x in (s, o):
+        x.load_state(f.reshape(-1), g.reshape(-1), None)
+        x.step(1)
+    for a, b in zip(s.fg(), o.fg()):
+        a, b = a.reshape(27, -1), b.reshape(27, -1)
+        assert np.all(np.abs(a - b) <= 5e-15 * _around(b, 1))
