@@ -65,3 +65,31 @@ def test_density_over_the_denominator_of_the_scalar_source(lib_built, oracle_mod
     for a, b in zip(s.fg(), o.fg()):
         a, b = a.reshape(27, -1), b.reshape(27, -1)
         assert np.all(np.abs(a - b) <= 5e-15 * _around(b, 1))
+
+
+# Populations from 2^16 on, and coefficients of that size, take the plain FP64 path, f and g each by itself.
+# "pair": the value at +x and at -x of one node, so that its velocity stays small and its coefficients below
+# the limit.  "single": at +x alone; the coefficient 9 u^2 / (216 tau) reaches 2^16 near u = 1.2e3.
+@pytest.mark.parametrize("node", [MIDDLE, WALL])
+@pytest.mark.parametrize("kind,which,value", [
+    ("pair", w, v) for w in (0, 1) for v in (2.0 ** 15, np.nextafter(2.0 ** 16, 0), 2.0 ** 16, 2.0 ** 17, 2.0 ** 19)] + [
+    ("single", 0, v) for v in (90.0, 1100.0, 1300.0, 2.0 ** 15)] + [
+    ("single", 1, v) for v in (2.0 ** 15, np.nextafter(2.0 ** 16, 0), 2.0 ** 16, 2.0 ** 17)])
+def test_both_sides_of_the_grids_limit_node_by_node(lib_built, oracle_mod, kind, which, value, node):
+    """A node's populations carry some ten roundings of 2^-53 of the largest term of the node they come from, so the
+    first (even) step lies within 5e-15 of the largest |f| around; the second (odd) one doubles the relative error
+    of u in u^2 and meets the first one's in k1: 4 times that.  Nodes out of reach of the value are compared with
+    what is around them alone, so they may not notice it."""
+    cfg = W.config("plain_fp64", lx=LX, ly=LY, lz=LZ)
+    fg = _populations(cfg, 8)
+    for d in (1, 3) if kind == "pair" else (1,):
+        fg[which][d, node] = value
+    s, o = Solver(cfg), oracle_mod.Oracle(cfg)
+    for x in (s, o):
+        x.load_state(fg[0].reshape(-1), fg[1].reshape(-1), None)
+    for step in (1, 2):
+        s.step(1, macros_last=True)
+        o.step(1)
+        for a, b in zip(s.fg(), o.fg()):
+            a, b = a.reshape(27, -1), b.reshape(27, -1)
+            assert np.all(np.abs(a - b) <= 5e-15 * 4 ** (step - 1) * _around(b, 1))
