@@ -186,15 +186,13 @@ int import_state(rbtp_handle *h, const double *f, const double *g, const double 
 {
     const long long L = h->geo.L;
     const size_t P = 27 * (size_t)L * sizeof(double), F7 = 7 * (size_t)L * sizeof(double);
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
     void *fs = h->f, *gs = h->g;
     const double *df = static_cast<const double *>(device_view(h, f, P));
     const double *dg = static_cast<const double *>(device_view(h, g, P));
     const double *d7 = flow7 ? static_cast<const double *>(device_view(h, flow7, F7)) : nullptr;
     if (df && dg && (!flow7 || d7)) {
         CK(launch_import_nodes(h->mode, h->geo, h->ph, 0, L, df, dg, L, d7, L, fs, gs, h->faux,
-                               h->rho, h->ux, h->uy, h->uz, h->phi, h->ted, h->ked, sms, h->stream));
+                               h->rho, h->ux, h->uy, h->uz, h->phi, h->ted, h->ked, h->sms, h->stream));
         return RBTP_OK;
     }
     // staged: chunks of C nodes, slot = f[27][C], g[27][C], flow7[7][C]
@@ -235,7 +233,7 @@ int import_state(rbtp_handle *h, const double *f, const double *g, const double 
         if (e == cudaSuccess) e = cudaStreamWaitEvent(h->stream, ev[b], 0);
         if (e == cudaSuccess)
             e = launch_import_nodes(h->mode, h->geo, h->ph, n0, cnt, sf, sg, C, flow7 ? s7 : nullptr, C, fs, gs,
-                                    h->faux, h->rho, h->ux, h->uy, h->uz, h->phi, h->ted, h->ked, sms, h->stream);
+                                    h->faux, h->rho, h->ux, h->uy, h->uz, h->phi, h->ted, h->ked, h->sms, h->stream);
         if (e == cudaSuccess) e = cudaEventRecord(ev[2 + b], h->stream);
     }
     // the staging slots are released only once every import has run
@@ -397,6 +395,7 @@ int rbtp_create(const rbtp_config *cfg, rbtp_handle **out)
             return cleanup_fail(e_ == cudaErrorMemoryAllocation ? RBTP_ERR_OOM : RBTP_ERR_CUDA); } \
     } while (0)
 
+    CKC(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device));
     CKC(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     {
         CKC(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
@@ -658,7 +657,7 @@ int rbtp_step_ex(rbtp_handle *h, int nsteps, unsigned flags)
         b.faux = h->faux; b.rho_wall = h->rho_wall;
         b.rho = h->rho; b.ux = h->ux; b.uy = h->uy; b.uz = h->uz; b.phi = h->phi;
         b.fcol = h->fcol; b.gcol = h->gcol; b.status = h->status;
-        CK(launch_step(h->mode, odd, out, h->geo, h->ph, b, h->stream));
+        CK(launch_step(h->mode, odd, out, h->geo, h->ph, b, h->sms, h->stream));
         if (parts) {
             // Stream order: the contacts (positions only) run on the side stream beside IBB
             // (latency-bound, few CTAs); the integrator waits for the contact forces.  The new link

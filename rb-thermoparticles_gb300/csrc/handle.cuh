@@ -23,6 +23,7 @@ struct rbtp_handle {
     Phys ph;
     int mode = RBTP_STORE_F64;
     int device = 0;
+    int sms = 1;                        // multiprocessors of the device
     cudaStream_t stream = nullptr;
     // particle steps: side stream for the contacts, which run beside IBB, with its fork/join events
     cudaStream_t side = nullptr;

@@ -273,7 +273,7 @@ inline unsigned lin_blocks(long long n, int t) { return (unsigned)((n + t - 1) /
 
 template <int MODE>
 cudaError_t launch_step_mode(bool odd, int out, const Geo &geo, const Phys &ph,
-                             const StepBuffers &b, cudaStream_t st)
+                             const StepBuffers &b, int sms, cudaStream_t st)
 {
     // FP64: one warp pair per block (step_node64.cuh).  FP32: warps of 32 x-nodes in one row (16-wide
     // blocks cost 3 % at 320x320x160, wider ones nothing).  Shifted FP16 is issue-bound: its odd steps use
@@ -287,19 +287,11 @@ cudaError_t launch_step_mode(bool odd, int out, const Geo &geo, const Phys &ph,
         if (out == OUT_MACROS_COL)
             return odd ? pdl_launch(k_step64<true, OUT_MACROS_COL, 1>, grd, blk, st, geo, ph, b, out)
                        : pdl_launch(k_step64<false, OUT_MACROS_COL, 1>, grd, blk, st, geo, ph, b, out);
-        // A grid of up to four waves of resident blocks runs at the latency of a block's chain of
-        // instructions, which unrolled slabs and fixed outputs shorten; a longer one is bound by
-        // throughput, and then the 42 KB of the odd step (32 KB of the even one) with the loop stay in
-        // the instruction caches and its 58 KB (45 KB) without do not.  Short chain | loop: 32x32x16
-        // 9.7 | 10.3 us, 64x64x32 40.6 | 42.4, 72x72x36 56.8 | 57.5, but 80x80x40 79.3 | 77.6, 96x96x48
-        // 129.8 | 124.5, 320x320x160 4.34 | 3.99 ms.
-        const long long blocks = (long long)grd.x * grd.y;
-        constexpr long long WAVE = 152LL * STEP64_BLOCKS, WAVE_MOST = 152LL * STEP64_BLOCKS_MOST;
-        if (blocks <= 4 * WAVE) {
-            // More resident blocks with fewer registers where that saves a wave that is more than a
-            // quarter full (9 | 12 blocks: 48x48x24 21.4 | 19.9 us, 60x60x30 36.3 | 35.2; but 40x40x20 16.6 |
-            // 20.1, 56x56x28 29.0 | 30.5, 64x64x32 40.6 | 42.3).
-            const bool most = (blocks + WAVE_MOST - 1) / WAVE_MOST < (blocks - WAVE / 4 + WAVE - 1) / WAVE;
+        // Short chain | loop: 32x32x16 9.7 | 10.3 us, 64x64x32 40.6 | 42.4, 72x72x36 56.8 | 57.5, but 80x80x40
+        // 79.3 | 77.6, 96x96x48 129.8 | 124.5, 320x320x160 4.34 | 3.99 ms.  9 | 12 resident blocks: 48x48x24 21.4 |
+        // 19.9 us, 60x60x30 36.3 | 35.2; but 40x40x20 16.6 | 20.1, 56x56x28 29.0 | 30.5, 64x64x32 40.6 | 42.3.
+        const Step64Choice choice = step64_choice((long long)grd.x * grd.y, sms);
+        if (choice.unrolled) {
             auto launch = [&](auto O, auto B) {
                 constexpr int OUT = decltype(O)::value, BLOCKS = decltype(B)::value;
                 return odd ? pdl_launch(k_step64<true, OUT, 3, BLOCKS>, grd, blk, st, geo, ph, b, out)
@@ -309,8 +301,8 @@ cudaError_t launch_step_mode(bool odd, int out, const Geo &geo, const Phys &ph,
             constexpr std::integral_constant<int, OUT_RUNTIME> ANY{};
             constexpr std::integral_constant<int, STEP64_BLOCKS> FEW{};
             constexpr std::integral_constant<int, STEP64_BLOCKS_MOST> MOST{};
-            if (out == OUT_NONE) return most ? launch(NONE, MOST) : launch(NONE, FEW);
-            return most ? launch(ANY, MOST) : launch(ANY, FEW);
+            if (out == OUT_NONE) return choice.most ? launch(NONE, MOST) : launch(NONE, FEW);
+            return choice.most ? launch(ANY, MOST) : launch(ANY, FEW);
         }
         return odd ? pdl_launch(k_step64<true, OUT_RUNTIME, 1>, grd, blk, st, geo, ph, b, out)
                    : pdl_launch(k_step64<false, OUT_RUNTIME, 1>, grd, blk, st, geo, ph, b, out);
@@ -338,12 +330,12 @@ cudaError_t launch_step_mode(bool odd, int out, const Geo &geo, const Phys &ph,
 }  // namespace
 
 cudaError_t launch_step(int mode, bool odd, int out, const Geo &geo, const Phys &ph,
-                        const StepBuffers &b, cudaStream_t st)
+                        const StepBuffers &b, int sms, cudaStream_t st)
 {
     switch (mode) {
-    case RBTP_STORE_F64: return launch_step_mode<RBTP_STORE_F64>(odd, out, geo, ph, b, st);
-    case RBTP_STORE_F32: return launch_step_mode<RBTP_STORE_F32>(odd, out, geo, ph, b, st);
-    case RBTP_STORE_F16S: return launch_step_mode<RBTP_STORE_F16S>(odd, out, geo, ph, b, st);
+    case RBTP_STORE_F64: return launch_step_mode<RBTP_STORE_F64>(odd, out, geo, ph, b, sms, st);
+    case RBTP_STORE_F32: return launch_step_mode<RBTP_STORE_F32>(odd, out, geo, ph, b, sms, st);
+    case RBTP_STORE_F16S: return launch_step_mode<RBTP_STORE_F16S>(odd, out, geo, ph, b, sms, st);
     }
     return cudaErrorInvalidValue;
 }

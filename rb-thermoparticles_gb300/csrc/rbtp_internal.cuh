@@ -338,8 +338,9 @@ struct StepBuffers {
     DevStatus *status;
 };
 
+// sms: the device's multiprocessors
 cudaError_t launch_step(int mode, bool odd, int out, const Geo &geo, const Phys &ph,
-                        const StepBuffers &b, cudaStream_t st);
+                        const StepBuffers &b, int sms, cudaStream_t st);
 // Post-streaming populations f(n) (the reference's d_f / d_g after a step) from an array in
 // PHASE_SWAPPED, as FP64 home layout: the odd step's gather, walls included, without collision.
 cudaError_t launch_stream_export(int mode, const Geo &geo, const Phys &ph, const void *fin,

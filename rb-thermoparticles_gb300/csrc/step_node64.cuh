@@ -22,6 +22,22 @@ constexpr int STEP64_DOUBLES = (27 * 2 + STEP64_SWAP) * STEP64_NODES;
 // short grids (lbm_step.cu), and 8 batched (12 | 10 | 9 | 8 | 7 | 6: 1.35 | 1.20 | 1.19 | 1.15 | 1.17 | 1.27 ms).
 constexpr int STEP64_BLOCKS = 9, STEP64_BLOCKS_MOST = 12, STEP64_BLOCKS_BATCHED = 8;
 
+// Variant of the single-cavity kernel for a grid of `blocks` on a GPU of `sms` multiprocessors.
+struct Step64Choice {
+    bool unrolled, most;
+};
+// A grid of up to four waves of resident blocks runs at the latency of a block's chain of instructions,
+// which unrolled slabs and fixed outputs shorten; a longer one is bound by throughput, and then the
+// code with the loop stays in the instruction caches and the longer one without does not.  Within the
+// short ones more resident blocks with fewer registers where that saves a wave that is more than a
+// quarter full.  Measured figures in lbm_step.cu.
+constexpr Step64Choice step64_choice(long long blocks, long long sms)
+{
+    const long long wave = sms * STEP64_BLOCKS, wave_most = sms * STEP64_BLOCKS_MOST;
+    const bool unrolled = blocks <= 4 * wave;
+    return {unrolled, unrolled && (blocks + wave_most - 1) / wave_most < (blocks - wave / 4 + wave - 1) / wave};
+}
+
 // eight times the direction index of a place, for loops that are not unrolled, and dir_mask by places
 static __constant__ int c_place_dir8[27] = {200, 72, 168, 144, 32, 112, 208, 80, 176, 136, 24, 104, 48, 0, 40, 120, 8, 88, 192, 64, 160, 128, 16, 96, 184, 56, 152};
 __host__ __device__ constexpr unsigned place_mask(int axis, int sign)

@@ -1,5 +1,5 @@
-// The host side of fixed64.cuh and collide64.cuh behind C functions, for test_fx_host.py.
-#include "collide64.cuh"
+// The host side of fixed64.cuh, collide64.cuh and step_node64.cuh behind C functions, for test_fx_host.py.
+#include "step_node64.cuh"
 
 using namespace rbtp;
 
@@ -20,5 +20,11 @@ long long fxh_times(double k, double d, unsigned grid, int up)
 {
     const FxFactor f = fx_factor(k);
     return fx_times(f, d, fx_places(f, grid, up));
+}
+// bit 0: unrolled, bit 1: more resident blocks
+int fxh_choice(long long blocks, long long sms)
+{
+    const Step64Choice c = step64_choice(blocks, sms);
+    return (c.unrolled ? 1 : 0) | (c.most ? 2 : 0);
 }
 }

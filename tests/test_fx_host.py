@@ -25,7 +25,8 @@ def fxh(tmp_path_factory):
                    check=True)
     L = ctypes.CDLL(str(lib))
     D, U, I, LL = ctypes.c_double, ctypes.c_uint, ctypes.c_int, ctypes.c_longlong
-    for name, res, args in (("grid", U, [D]), ("from", LL, [D, U]), ("to", D, [LL, U, I]), ("times", LL, [D, D, U, I])):
+    for name, res, args in (("grid", U, [D]), ("from", LL, [D, U]), ("to", D, [LL, U, I]), ("times", LL, [D, D, U, I]),
+                            ("choice", I, [LL, LL])):
         fn = getattr(L, "fxh_" + name)
         fn.restype, fn.argtypes = res, args
     return L
@@ -97,3 +98,14 @@ def test_products_are_rounded_to_odd_on_the_grid(fxh):
             total += (got - want) * (1 if want > 0 else -1)
             n += 1
     assert abs(float(total / n)) < 4 * 3 ** -0.5 / n ** 0.5 + 2.0 ** -8
+
+
+@pytest.mark.parametrize("sms", [76, 132, 148, 152, 160])
+def test_variant_of_a_grid_follows_the_multiprocessor_count(fxh, sms):
+    """Four waves of nine resident blocks are the last unrolled grid; twelve are taken where ceil(blocks / 12 sms)
+    is below the waves of nine, of which the last counts from a quarter on."""
+    for blocks in [1, sms, *(k * sms * n + d for n in (9, 12) for k in (1, 2, 3, 4, 5) for d in (-1, 0, 1, 2 * sms, 3 * sms)), 10 ** 6]:
+        waves = -(-(blocks - 9 * sms // 4) // (9 * sms))
+        unrolled = blocks <= 36 * sms
+        most = unrolled and -(-blocks // (12 * sms)) < waves
+        assert fxh.fxh_choice(blocks, sms) == unrolled + 2 * most, blocks
