@@ -664,10 +664,12 @@ int rbtp_step_ex(rbtp_handle *h, int nsteps, unsigned flags)
             // slabs, which the next step's IBB takes, are filled beside the refill (with the
             // clears in one kernel: 64x64x32 with 9 spheres 103 -> 83 us per step in FP32 and
             // 153 -> 128 in FP64, 1000 spheres in FP32 1.73 -> 1.71 ms), but not beside the next
-            // HBM-bound bulk kernel, whose SM slots their CTAs would take (measured slower).  The
-            // particle kernels use ordinary launches: programmatic dependent launch, which lets
-            // each one's blocks become resident while its predecessor finishes, made the
-            // 1000-sphere step 0.3 % (FP32) and 0.6 % (FP64) slower.
+            // HBM-bound bulk kernel, whose SM slots their CTAs would take (measured slower).
+            // Below 608 spheres (chained() in particles.cu) IBB, the cell scan and fill, the contact
+            // forces, the marking and the refill's scatter are launched with programmatic dependence: their
+            // blocks may become resident while the kernel before them in their stream finishes, and each
+            // waits for its end before it touches memory.  All other kernels, and all from 608 spheres on
+            // (1.669 against 1.682 ms per step with 1000 in FP32), start when their predecessor is done.
             int *oc = h->owner[h->ocur], *on = h->owner[1 - h->ocur];
             CK(launch_step_clear(h->geo, h->pb, on, h->status, h->stream));
             CK(cudaEventRecord(h->ev_fork, h->stream));

@@ -19,7 +19,7 @@
 // which are frequent, since many members are only a few places below the largest.  Closed 16x12x8
 // cavities at Ra 2e4 and 1e5, mass after 20,000 steps: 1.2e-15 and 4e-15 (9e-15 and -4e-15 with FP64
 // formulas; -2.4e-12 and -3.1e-12 with members cut off, 3e-13 and -3e-13 with ties away from zero).  At
-// 320x320x160 the step takes 4.45 ms, 4.0 with members cut off, 4.76 with members to nearest.
+// 320x320x160 the step took 4.00 ms with members cut off, 4.45 with them rounded to odd, 4.76 to nearest.
 // Conversions work on sign and magnitude, so the arithmetic is exactly odd: negated inputs give
 // negated results, and zeros stay zeros.  Room: 53 + FX_GUARD bits of a member leave a factor of 31 for
 // the sum.

@@ -287,9 +287,10 @@ cudaError_t launch_step_mode(bool odd, int out, const Geo &geo, const Phys &ph,
         if (out == OUT_MACROS_COL)
             return odd ? pdl_launch(k_step64<true, OUT_MACROS_COL, 1>, grd, blk, st, geo, ph, b, out)
                        : pdl_launch(k_step64<false, OUT_MACROS_COL, 1>, grd, blk, st, geo, ph, b, out);
-        // Short chain | loop: 32x32x16 9.7 | 10.3 us, 64x64x32 40.6 | 42.4, 72x72x36 56.8 | 57.5, but 80x80x40
-        // 79.3 | 77.6, 96x96x48 129.8 | 124.5, 320x320x160 4.34 | 3.99 ms.  9 | 12 resident blocks: 48x48x24 21.4 |
-        // 19.9 us, 60x60x30 36.3 | 35.2; but 40x40x20 16.6 | 20.1, 56x56x28 29.0 | 30.5, 64x64x32 40.6 | 42.3.
+        // Short chain | loop: 32x32x16 10.4 | 11.1 us, 64x64x32 (3.0 waves) 44.2 | 45.8, 72x72x36 (4.3, the slower
+        // one by the rule) 62.0 | 62.5, but 80x80x40 (5.8) 86.3 | 83.8, 96x96x48 142.9 | 136.9, 320x320x160 4.90 |
+        // 4.38 ms.  9 | 12 resident blocks: 48x48x24 23.3 | 21.7 us, 60x60x30 39.8 | 38.7; but 40x40x20 17.8 | 21.6,
+        // 56x56x28 31.9 | 33.2, 64x64x32 44.2 | 47.1.
         const Step64Choice choice = step64_choice((long long)grd.x * grd.y, sms);
         if (choice.unrolled) {
             auto launch = [&](auto O, auto B) {

@@ -17,9 +17,10 @@ constexpr int STEP64_NODES = 32;
 constexpr int STEP64_SWAP = 16;      // doubles exchanged per node
 constexpr int STEP64_DOUBLES = (27 * 2 + STEP64_SWAP) * STEP64_NODES;
 // Resident blocks per SM that the kernels ask registers for: 9 (up to 112 per thread), the best of 8 to 12 where a
-// grid has several waves (320x320x160 at 12 | 11 | 10 | 9 | 8: 4.21 | 4.17 | 4.11 | 3.99 | 4.26 ms per step;
-// 113x97x59 196 | 195 | 177 | 173 | 184 us), 12 (80 per thread, all that shared memory allows) for some
-// short grids (lbm_step.cu), and 8 batched (12 | 10 | 9 | 8 | 7 | 6: 1.35 | 1.20 | 1.19 | 1.15 | 1.17 | 1.27 ms).
+// grid has several waves (320x320x160 at 12 | 11 | 10 | 9 | 8: 4.66 | 4.64 | 4.42 | 4.38 | 4.90 ms per step;
+// 113x97x59 212 | 211 | 190 | 191 | 205 us), 12 (80 per thread, all that shared memory allows) for some
+// short grids (lbm_step.cu), and 8 batched (12 | 11 | 10 | 9 | 8 | 7: 1.44 | 1.44 | 1.33 | 1.33 | 1.30 | 1.31 ms
+// for 32 members of 32 to 96 nodes across).
 constexpr int STEP64_BLOCKS = 9, STEP64_BLOCKS_MOST = 12, STEP64_BLOCKS_BATCHED = 8;
 
 // Variant of the single-cavity kernel for a grid of `blocks` on a GPU of `sms` multiprocessors.
@@ -112,11 +113,11 @@ __device__ __forceinline__ double *slot_at(double *base, unsigned i8, unsigned L
 // warps fit a scheduler; the populations therefore go from global to shared memory by cp.async, without
 // passing through registers, and are read from there where they are used, and f and g of a node
 // belong to two threads, which exchange the moments: four and a half warps per scheduler.  The code loops over the
-// three slabs of directions: unrolled, its 75 KB did not stay in the instruction caches.  Measured
-// at 320x320x160: 4.0 ms per step, 13.1 ms with every sum on the FP64 pipe (424 FP64 instructions
-// per node there, 77 here; 880 B per node at the copy bandwidth would take 2.2 ms); at 64x64x32 41
+// three slabs of directions: unrolled, it did not stay in the instruction caches (4.90 ms).  Measured
+// at 320x320x160: 4.38 ms per step, 13.1 ms with every sum on the FP64 pipe (424 FP64 instructions
+// per node there, 77.4 here; 880 B per node at the copy bandwidth would take 2.2 ms); at 64x64x32 44
 // against 118 us.  What bounds it now is the latency of the chain load - integer sums - FP64
-// coefficients - integer sums with the warps that fit (issue slots 62 %, integer pipe 68 %, FP64 pipe 50 % busy).  `out`
+// coefficients - integer sums with the warps that fit (issue slots 60 %, integer pipe 70 %, FP64 pipe 46 % busy).  `out`
 // selects the outputs (StepOut; COL: also the post-collision copies; a kernel for each value had the
 // compiler unroll some, see the choice of UNROLL, the slabs per round of the collision's loop, in
 // lbm_step.cu), `smem` is the block's shared memory.  Threads that are not `active` only take part in

@@ -1,6 +1,6 @@
 """The FP64 step's integer-unit sums at the edges of their ranges: row remainders of the 32-node warps,
-populations from 2^-300 to 2^80 within a node, values beyond the grids (the plain FP64 path), and
-non-finite ones.  Against the oracle's plain FP64 formulas; the tolerance is a few roundings (2^-53
+populations 2^-300 to 1 times their size within a node, values far beyond the grids' limit of 2^16 (the
+plain FP64 path), and non-finite ones.  Against the oracle's plain FP64 formulas; the tolerance is a few roundings (2^-53
 each) of the node's largest terms per step, over at most four steps."""
 import numpy as np
 import pytest
